@@ -29,12 +29,29 @@ constexpr int kBlockThreads = 256;  // default transport block size (the autotun
 // Fixed-point scale of the energy tally: edep is accumulated as int64 multiples of 2^-32 MeV.
 constexpr double kEdepScale = 4294967296.0;
 
+// Values for which the transport kernel's quotient() (reciprocal + fused
+// multiply-adds instead of a division) is proven: no overflow, no subnormal
+// remainder for the operands transport divides.
+constexpr float kQuotientMin = 1.0e-25f, kQuotientMax = 1.0e25f;
+constexpr uint32_t kPackCount = 0x7fu, kPackReciprocals = 0x80u;
+// Voxel index of a solid: general (divisions, integer conversions),
+// multiplication by an exact 2^-k, or quotient() with the correctly rounded
+// reciprocal; the last two for at most 2^22 voxels an axis (trunc by rounding
+// at 2^23).  A box is a grid of one voxel: reciprocal 0, so that every position
+// has index 0.  A launch takes the first of general, reciprocal, pow2 that one
+// of its solids needs.
+constexpr int kVoxelGeneral = 0, kVoxelPow2 = 1, kVoxelReciprocal = 2, kVoxelBox = 3;
+// Tables with reciprocals may take this much of a block's shared memory: three
+// blocks of 256 threads with the photon stash stay resident per SM.  Larger
+// ones keep plain rows and divide.
+constexpr uint32_t kReciprocalTableBytes = 44 * 1024;
+
 struct alignas(16) DevNavigator {
   // read by every tracking step: the first 16 bytes, one vector load
   int32_t number_of_bins;
-  uint32_t process_pack;         // number_of_processes | process_id[0] << 8 | process_id[1] << 16 | process_id[2] << 24
+  uint32_t process_pack;         // number_of_processes (kPackCount) | kPackReciprocals | process_id[i] << 8 (i + 1)
   // byte offsets into the table blob (shared memory copy when it fits)
-  uint32_t sigma_offset;         // float4[number_of_materials * number_of_bins]
+  uint32_t sigma_offset;         // float4[number_of_materials * number_of_bins] (or [...][2] with the reciprocals)
   uint32_t photon_cut_offset;    // float[number_of_materials]
   int32_t number_of_materials;
   int32_t number_of_processes;
@@ -68,12 +85,12 @@ struct alignas(16) DevSolid {
   float border_min[3];
   float border_max[3];
   float voxel_sizes[3];
-  float inv_voxel_sizes[3];      // exact 2^-k when voxel_pow2
+  float inv_voxel_sizes[3];      // 1 / voxel_sizes correctly rounded (exact for powers of two)
   int32_t number_of_voxels[3];
   int32_t navigator;
   const uint8_t* labels;
   int32_t type;
-  int32_t voxel_pow2;            // every voxel size is a power of two
+  int32_t voxel_mode;            // how the voxel index divides by the voxel size (kVoxel*)
   float matrix[16];
   float threshold;
   int32_t virtual_element_number[3];
@@ -168,6 +185,10 @@ struct TransportParams {
   int32_t tracking_capacity;
   gg_track_point* tracking_points;
   int32_t* tracking_count;
+  int32_t voxel_mode;               // kVoxelGeneral, kVoxelReciprocal or kVoxelPow2: what serves every solid of the launch
+  int32_t fast_sampling;            // every navigator: all three processes, sigma rows with reciprocals
+  int32_t photon_tracking;          // some dose map counts photons
+  int32_t tle;                      // some dose map uses the track-length estimator
   int32_t regroup_lanes;            // waiting lanes that start a round of the rare phases (1..32)
   int32_t regroup_ratio4;           // ... or 4 x waiting >= regroup_ratio4 x tracking lanes
   uint32_t slots_per_claim;         // consecutive slots a lane takes from the work queue at a time (power of two)

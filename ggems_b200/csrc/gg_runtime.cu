@@ -106,6 +106,8 @@ struct gg_context {
   unsigned char* table_blob = nullptr;
   uint32_t table_bytes = 0;
   bool tables_in_smem = false;
+  uint8_t* zero_label = nullptr;  // material 0: the one voxel of a detector box
+  std::vector<uint32_t> process_pack;  // per navigator, as uploaded
   unsigned int* slot_counter = nullptr;
   int* error = nullptr;
   cudaEvent_t start = nullptr, stop = nullptr;
@@ -413,15 +415,29 @@ int make_dev_solid(gg_context* c, const gg_solid& g, gg::DevSolid* out, std::vec
   d.threshold = g.threshold;
   std::memcpy(d.number_of_voxels, g.number_of_voxels, sizeof(d.number_of_voxels));
   std::memcpy(d.voxel_sizes, g.voxel_sizes, sizeof(d.voxel_sizes));
-  // x / 2^k and x * 2^-k are the same correctly rounded value for every x,
-  // so power-of-two voxel sizes let the kernel multiply instead of divide.
-  d.voxel_pow2 = 1;
+  // x / 2^k and x * 2^-k are the same correctly rounded value for every x, so
+  // power-of-two voxel sizes let the kernel multiply instead of divide; other
+  // sizes take the reciprocal form of the same quotient.
+  bool pow2 = true, reciprocal = true;
   for (int a = 0; a < 3; ++a) {
     int e = 0;
-    const float m = std::frexp(g.voxel_sizes[a], &e);  // v = m * 2^e, m in [0.5, 1)
-    const bool pow2 = std::isfinite(g.voxel_sizes[a]) && m == 0.5f && e > -125 && e < 127;
-    d.voxel_pow2 &= pow2 ? 1 : 0;
-    d.inv_voxel_sizes[a] = pow2 ? std::ldexp(1.0f, 1 - e) : 0.0f;
+    const float v = g.voxel_sizes[a];
+    const float m = std::frexp(v, &e);  // v = m * 2^e, m in [0.5, 1)
+    pow2 &= std::isfinite(v) && m == 0.5f;
+    reciprocal &= v >= gg::kQuotientMin && v <= gg::kQuotientMax && g.number_of_voxels[a] <= (1 << 22);
+    d.inv_voxel_sizes[a] = 1.0f / v;
+  }
+  d.voxel_mode = !reciprocal ? gg::kVoxelGeneral : (pow2 ? gg::kVoxelPow2 : gg::kVoxelReciprocal);
+  if (g.type == GG_SOLID_BOX) {
+    // one voxel of material 0, where that reproduces the borders bit for bit
+    bool same = true;
+    for (int a = 0; a < 3; ++a) {
+      d.number_of_voxels[a] = 1;
+      d.voxel_sizes[a] = d.border_max[a] - d.border_min[a];
+      d.inv_voxel_sizes[a] = 0.0f;
+      same &= d.border_min[a] + d.voxel_sizes[a] == d.border_max[a];
+    }
+    d.voxel_mode = same ? gg::kVoxelBox : gg::kVoxelGeneral;
   }
   std::memcpy(d.virtual_element_number, g.virtual_element_number, sizeof(d.virtual_element_number));
   std::memcpy(d.box_size, g.box_size, sizeof(d.box_size));
@@ -449,7 +465,9 @@ int make_dev_solid(gg_context* c, const gg_solid& g, gg::DevSolid* out, std::vec
     }
   } else if (g.type == GG_SOLID_MESHED) {
     if ((rc = upload_mesh(c, g, &d, owner))) return rc;
-  } else if (g.type != GG_SOLID_BOX) {
+  } else if (g.type == GG_SOLID_BOX) {
+    d.labels = c->zero_label;
+  } else {
     return fail(GG_ERROR_INVALID_ARGUMENT, "solid type not supported by this build");
   }
   return GG_OK;
@@ -521,6 +539,8 @@ GG_API int gg_context_create(int32_t device_index, gg_context** context) {
   if (cudaMalloc(&c->particles.status, S) != cudaSuccess || cudaMalloc(&c->particles.scatter, S) != cudaSuccess ||
       cudaMalloc(&c->particles.solid_id, S * sizeof(int32_t)) != cudaSuccess)
     return cleanup(fail(GG_ERROR_OUT_OF_MEMORY, "particles"));
+  if (cudaMalloc(&c->zero_label, 16) != cudaSuccess || cudaMemset(c->zero_label, 0, 16) != cudaSuccess)
+    return cleanup(fail(GG_ERROR_OUT_OF_MEMORY, "labels"));
   if (cudaMalloc(&c->slot_counter, sizeof(unsigned int)) != cudaSuccess ||
       cudaMalloc(&c->error, sizeof(int)) != cudaSuccess)
     return cleanup(fail(GG_ERROR_OUT_OF_MEMORY, "counters"));
@@ -549,6 +569,7 @@ GG_API int gg_context_destroy(gg_context* c) {
   cudaFree(c->particles.status);
   cudaFree(c->particles.scatter);
   cudaFree(c->particles.solid_id);
+  cudaFree(c->zero_label);
   cudaFree(c->slot_counter);
   cudaFree(c->error);
   if (c->dose_out) cudaFree(c->dose_out);
@@ -620,6 +641,25 @@ GG_API int gg_upload_scene(gg_context* c, const gg_scene* sc) {
       nav_tle[g.navigator] = 1;
   }
 
+  // Rows with reciprocals: every cross section 0 or within quotient()'s range,
+  // and the whole set small enough (kReciprocalTableBytes).
+  bool with_reciprocals = true;
+  size_t reciprocal_bytes = 0;
+  for (int n = 0; n < sc->number_of_tables && with_reciprocals; ++n) {
+    const gg_physics_tables& t = sc->tables[n];
+    const size_t cells = static_cast<size_t>(std::max(t.number_of_materials, 0)) * std::max(t.number_of_bins, 0);
+    reciprocal_bytes += cells * 32 + static_cast<size_t>(std::max(t.number_of_bins, 0)) * 4;
+    if (nav_tle[n]) reciprocal_bytes += (1 + static_cast<size_t>(std::max(t.number_of_materials, 0))) * GG_ATTENUATION_BINS * 4;
+    with_reciprocals = reciprocal_bytes <= gg::kReciprocalTableBytes;
+    for (int p = 0; p < std::min(t.number_of_processes, 3) && with_reciprocals; ++p) {
+      if (t.process_id[p] < 0 || t.process_id[p] > 2) break;  // refused below
+      for (size_t i = 0; i < cells && with_reciprocals; ++i) {
+        const float s = t.cross_sections[t.process_id[p] * cells + i];
+        with_reciprocals = s == 0.0f || (s >= gg::kQuotientMin && s <= gg::kQuotientMax);
+      }
+    }
+  }
+
   // ---- tables: shared-memory blob + HBM element data ----
   std::vector<unsigned char> blob;
   std::vector<gg::DevNavigator> navs(sc->number_of_tables);
@@ -643,12 +683,18 @@ GG_API int gg_upload_scene(gg_context* c, const gg_scene* sc) {
     blob.resize(align16(d.energy_bins_offset + nb * 4), 0);
     std::memcpy(blob.data() + d.energy_bins_offset, t.energy_bins, nb * 4);
     d.sigma_offset = static_cast<uint32_t>(blob.size());
-    blob.resize(d.sigma_offset + nm * nb * 16, 0);
+    blob.resize(d.sigma_offset + nm * nb * (with_reciprocals ? 32 : 16), 0);
     float* sig = reinterpret_cast<float*>(blob.data() + d.sigma_offset);
     const size_t block = static_cast<size_t>(nm) * nb;
+    const uint32_t row = with_reciprocals ? 8 : 4;
     for (uint32_t m = 0; m < nm; ++m)
       for (uint32_t b = 0; b < nb; ++b)
-        for (int p = 0; p < 3; ++p) sig[(m * nb + b) * 4 + p] = t.cross_sections[p * block + b + nb * m];
+        for (int p = 0; p < t.number_of_processes; ++p) {
+          const float s = t.cross_sections[t.process_id[p] * block + b + nb * m];
+          sig[(m * nb + b) * row + p] = s;
+          if (with_reciprocals) sig[(m * nb + b) * row + 4 + p] = 1.0f / s;
+        }
+    if (with_reciprocals) d.process_pack |= gg::kPackReciprocals;
     d.photon_cut_offset = static_cast<uint32_t>(blob.size());
     blob.resize(align16(d.photon_cut_offset + nm * 4), 0);
     std::memcpy(blob.data() + d.photon_cut_offset, t.photon_energy_cut, nm * 4);
@@ -694,6 +740,8 @@ GG_API int gg_upload_scene(gg_context* c, const gg_scene* sc) {
   int rc;
   if ((rc = dev_copy(c, blob.data(), blob.size(), &c->table_blob))) return rc;
   if ((rc = dev_copy(c, navs.data(), navs.size(), &c->navigators))) return rc;
+  c->process_pack.clear();
+  for (const gg::DevNavigator& d : navs) c->process_pack.push_back(d.process_pack);
   c->number_of_navigators = sc->number_of_tables;
 
   // ---- tallies ----
@@ -945,6 +993,17 @@ int prepare_jobs(gg_context* c, const gg_job* jobs, int32_t n, std::vector<void*
   P.tables_in_smem = c->tables_in_smem ? 1 : 0;
   P.slot_counter = c->slot_counter;
   P.error = c->error;
+  P.voxel_mode = gg::kVoxelPow2;
+  auto need_mode = [&](const gg::DevSolid& d) {
+    if (d.type == GG_SOLID_MESHED || d.voxel_mode == gg::kVoxelBox || P.voxel_mode == gg::kVoxelGeneral) return;
+    if (d.voxel_mode != gg::kVoxelPow2) P.voxel_mode = d.voxel_mode;
+  };
+  for (int s = 0; s < c->number_of_solids; ++s) need_mode(c->solid_dev_host[s]);
+  for (const gg::DevSolid& d : job_solids) need_mode(d);
+  P.fast_sampling = 1;
+  for (uint32_t pack : c->process_pack) P.fast_sampling &= (pack & 0xffu) == (3u | gg::kPackReciprocals) ? 1 : 0;
+  for (const gg::DevDoseMap& m : c->dose_host) P.photon_tracking |= m.photon_tracking ? 1 : 0;
+  for (char t : c->dose_tle) P.tle |= t ? 1 : 0;
   P.regroup_lanes = c->regroup_lanes;
   P.regroup_ratio4 = c->regroup_ratio4;
   P.slots_per_claim = static_cast<uint32_t>(c->slots_per_claim);

@@ -52,6 +52,16 @@ constexpr float kRayleighFactor = 32526509815670243328.0f;  // GGEMSRayleighScat
 constexpr float kKissTwoToMinus32 = 0x1p-32f;
 constexpr float kKissCorrection = -0x1.ffp-56f;  // -(2^-23 - 2^-32) * 2^-32, exact in float
 
+// Tracking steps a lane takes between two looks at its warp's waiting photons.
+// The look (ballots, counts, the stash's exchange test) costs every lane about
+// as much as a fifth of a step; a lane that stops early idles for the rest.
+// Without dose maps 1 / 2 / 4 / 8 steps: CBCT 33.4 / 32.0 / 30.4 / 29.9 ms per
+// 1e7 primaries, 36 projections of 1e6 31.6 / 30.3 / 28.0 / 26.5 ms.  With dose
+// maps the steps diverge at their tallies: C1 water 1.20 ms at 2 and 1.22 to
+// 1.23 at 1 and 3, TLE emission 11.2 at 2, 11.7 and 12.1.
+constexpr int kTrackSteps = 8, kTrackStepsDose = 2;
+constexpr float kTwo23 = 8388608.0f;
+
 enum Phase : int { kNewHistory = 0, kFind = 1, kTrackVoxel = 2, kTrackBox = 3, kTrackMesh = 4, kInteract = 5, kDone = 6 };
 
 struct V3 {
@@ -143,52 +153,40 @@ __device__ __forceinline__ bool in_aabb(V3 p, V3 mn, V3 mx) {
 }
 // inv holds 1.0f / d per axis (used only where |d| >= 1e-6, as the reference
 // computes it there), so a direction's reciprocals can be computed once.
+// The reference's early returns all give kOutOfWorld and its running
+// tmin <= tmax test can only fail for good (tmin grows, tmax shrinks), so the
+// axes are combined without branches and tested once at the end.  (A branch for
+// the rare direction along a face instead of the selects: CBCT 33.7 against
+// 31.3 ms per 1e7 primaries.)
 __device__ __forceinline__ float distance_to_aabb(V3 p, V3 d, V3 inv, V3 mn, V3 mx) {
   float tmin = FLT_MIN, tmax = FLT_MAX;
-  if (fabsf(d.x) < kEps6) {
-    if (p.x < mn.x || p.x > mx.x) return kOutOfWorld;
-  } else {
-    float id = inv.x;
-    tmin = (mn.x - p.x) * id;
-    tmax = (mx.x - p.x) * id;
-    if (tmin > tmax) {
-      float t = tmin;
-      tmin = tmax;
-      tmax = t;
-    }
+  bool miss = false;
+  {
+    const float a = (mn.x - p.x) * inv.x, b = (mx.x - p.x) * inv.x;
+    const bool along = fabsf(d.x) < kEps6;
+    miss = along && (p.x < mn.x || p.x > mx.x);
+    tmin = along ? tmin : fminf(a, b);
+    tmax = along ? tmax : fmaxf(a, b);
   }
-  if (fabsf(d.y) < kEps6) {
-    if (p.y < mn.y || p.y > mx.y) return kOutOfWorld;
-  } else {
-    float id = inv.y;
-    float lo = (mn.y - p.y) * id, hi = (mx.y - p.y) * id;
-    if (lo > hi) {
-      float t = lo;
-      lo = hi;
-      hi = t;
-    }
-    if (lo > tmin) tmin = lo;
-    if (hi < tmax) tmax = hi;
-    if (tmin > tmax) return kOutOfWorld;
+  {
+    const float a = (mn.y - p.y) * inv.y, b = (mx.y - p.y) * inv.y;
+    const bool along = fabsf(d.y) < kEps6;
+    miss = miss || (along && (p.y < mn.y || p.y > mx.y));
+    tmin = along ? tmin : fmaxf(tmin, fminf(a, b));
+    tmax = along ? tmax : fminf(tmax, fmaxf(a, b));
   }
-  if (fabsf(d.z) < kEps6) {
-    if (p.z < mn.z || p.z > mx.z) return kOutOfWorld;
-  } else {
-    float id = inv.z;
-    float lo = (mn.z - p.z) * id, hi = (mx.z - p.z) * id;
-    if (lo > hi) {
-      float t = lo;
-      lo = hi;
-      hi = t;
-    }
-    if (lo > tmin) tmin = lo;
-    if (hi < tmax) tmax = hi;
-    if (tmin > tmax) return kOutOfWorld;
+  {
+    const float a = (mn.z - p.z) * inv.z, b = (mx.z - p.z) * inv.z;
+    const bool along = fabsf(d.z) < kEps6;
+    miss = miss || (along && (p.z < mn.z || p.z > mx.z));
+    tmin = along ? tmin : fmaxf(tmin, fminf(a, b));
+    tmax = along ? tmax : fminf(tmax, fmaxf(a, b));
   }
-  if (tmin < 0.0f && (tmax < 0.0f || tmax == 0.0f)) return kOutOfWorld;
-  if (static_cast<double>(tmax - tmin) < (2.0 * static_cast<double>(kTolerance))) return kOutOfWorld;
-  if (tmin <= kEps6) return tmax;
-  return tmin;
+  miss = miss || tmin > tmax || (tmin < 0.0f && tmax <= 0.0f);
+  // the reference compares in double; 2 x kTolerance is exact in float
+  miss = miss || (tmax - tmin) < 2.0f * kTolerance;
+  const float t = tmin <= kEps6 ? tmax : tmin;
+  return miss ? kOutOfWorld : t;
 }
 
 __device__ __forceinline__ V3 reciprocal(V3 d) { return v3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z); }
@@ -241,29 +239,70 @@ struct Tab {
   }
 };
 
-__device__ __forceinline__ float pick(float4 s, int pid) { return pid == 0 ? s.x : (pid == 1 ? s.y : s.z); }
+__device__ __forceinline__ float pick(float4 s, int i) { return i == 0 ? s.x : (i == 1 ? s.y : s.z); }
+
+// a / b correctly rounded from y = the correctly rounded 1 / b, without the
+// division instruction sequence's branch to its slow path: one refinement makes
+// the quotient faithful, the second is Markstein's final step (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// IBM J. Res. Dev. 34 (1990): a faithful q and a correctly rounded y give
+// RN(q + y RN(a - b q)) = RN(a / b)).  Needs exponents away from the ends of
+// the range, which the host checks (kQuotientMin / kQuotientMax) for b; b = 0
+// with y = inf gives NaN where a / b is inf (a > 0).
+__device__ __forceinline__ float quotient(float a, float b, float y) {
+  float q = a * y;
+  q = __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+  return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+}
 
 // GetPhotonNextInteraction, GGEMSPhotonNavigator.hh:57-93.  Returns the
-// distance, writes the process; energy_id is the cached BinarySearch result,
-// process_pack the navigator's process count and ids (DevNavigator).
-__device__ __forceinline__ float next_interaction(Kiss& rng, int number_of_bins, uint32_t process_pack,
-                                                  const float4* sig, int energy_id, int material, int& proc) {
-  float4 s = sig[material * number_of_bins + energy_id];
+// distance, writes the process; `row` is the sigma table's row of the material
+// and the cached BinarySearch result (process order; two float4 with the
+// reciprocals in the second when process_pack says so), process_pack the
+// navigator's process count and ids (DevNavigator).  fast: every navigator of
+// the launch has all three processes and reciprocals; then the three draws,
+// logarithms and quotients have no branch and overlap.  A cross section of 0
+// gives NaN there, which is not below nid, as the reference's infinite distance
+// is not.
+__device__ __forceinline__ float next_interaction(Kiss& rng, uint32_t process_pack, bool fast, const float4* row,
+                                                  int& proc) {
   float nid = kOutOfWorld;
+  const float4 s = row[0];
+  if (fast) {
+    const float4 y = row[1];
+    const float a0 = -logf(rng.uniform()), a1 = -logf(rng.uniform()), a2 = -logf(rng.uniform());
+    const float d0 = quotient(a0, s.x, y.x), d1 = quotient(a1, s.y, y.y), d2 = quotient(a2, s.z, y.z);
+    int shift = 0;
+    if (d0 < nid) {
+      nid = d0;
+      shift = 8;
+    }
+    if (d1 < nid) {
+      nid = d1;
+      shift = 16;
+    }
+    if (d2 < nid) {
+      nid = d2;
+      shift = 24;
+    }
+    proc = shift == 0 ? kNoProcess : static_cast<int>((process_pack >> shift) & 0xffu);
+    return nid;
+  }
   proc = kNoProcess;
-  const int n = static_cast<int>(process_pack & 0xffu);
+  const int n = static_cast<int>(process_pack & kPackCount);
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     if (i >= n) break;
-    const int pid = static_cast<int>((process_pack >> (8 * (i + 1))) & 0xffu);
-    float dist = -logf(rng.uniform()) / pick(s, pid);
+    const float dist = -logf(rng.uniform()) / pick(s, i);
     if (dist < nid) {
       nid = dist;
-      proc = pid;
+      proc = static_cast<int>((process_pack >> (8 * (i + 1))) & 0xffu);
     }
   }
   return nid;
 }
+// Float4s a row of the sigma table takes.
+__device__ __forceinline__ int row_stride(uint32_t process_pack) { return (process_pack & kPackReciprocals) ? 2 : 1; }
 
 // 16-byte shared-memory (or global) loads of a struct's leading fields.
 __device__ __forceinline__ float4 load4f(const void* p) { return *reinterpret_cast<const float4*>(p); }
@@ -345,8 +384,10 @@ __device__ __noinline__ Interaction rayleigh(Interaction in, const DevNavigator&
   int mixture = nv.element_offset[material];
   int z = nv.atomic_number[mixture + n_minus_one];
   if (n_minus_one > 0) {
-    float kcs = lerp_ref(ebins[energy_id], sig[material * nb + energy_id].z, ebins[energy_id + 1],
-                         sig[material * nb + energy_id + 1].z, E0);
+    const int stride = row_stride(nv.process_pack);
+    const float4* row = sig + static_cast<size_t>(material * nb + energy_id) * stride;
+    const int slot = nv.process_id[0] == GG_RAYLEIGH_SCATTERING ? 0 : (nv.process_id[1] == GG_RAYLEIGH_SCATTERING ? 1 : 2);
+    float kcs = lerp_ref(ebins[energy_id], pick(row[0], slot), ebins[energy_id + 1], pick(row[stride], slot), E0);
     float x = rng.uniform() * kcs;
     float cs = 0.0f;
     for (int i = 0; i < n_minus_one; ++i) {
@@ -1253,20 +1294,14 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
     if (phase != kTrackVoxel && phase != kTrackBox && !(kFull && phase == kTrackMesh)) continue;
     {
 
-    // ---- one tracking step inside solid ph.solid_id ----
+    // ---- tracking inside solid ph.solid_id ----
     // the solid's and navigator's per-step fields in six 16-byte loads
     // (DevSolid / DevNavigator lead with them)
     const DevSolid& so = solids[ph.solid_id];
-    const float4 s0 = load4f(&so.border_min[0]);     // border_min xyz, border_max x
-    const float4 s1 = load4f(&so.border_max[1]);     // border_max yz, voxel_sizes xy
-    const float4 s2 = load4f(&so.voxel_sizes[2]);    // voxel_sizes z, inv_voxel_sizes xyz
     const int4 s3 = load4i(&so.number_of_voxels[0]);  // number_of_voxels xyz, navigator
-    const int4 s4 = load4i(&so.labels);               // labels (2 words), type, voxel_pow2
     const int nav = s3.w;
     const int4 n0 = load4i(&navs[nav]);               // number_of_bins, process_pack, sigma / cut offsets
     const float4* sig = reinterpret_cast<const float4*>(tab.base + static_cast<uint32_t>(n0.z));
-    V3 bmin = v3(s0.x, s0.y, s0.z);
-    V3 bmax = v3(s0.w, s1.x, s1.y);
     if (ph.E != cached_E || nav != cached_nav) {
       energy_id = binary_search(ph.E, tab.energy_bins(nav), n0.x);
       cached_E = ph.E;
@@ -1274,22 +1309,57 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
     }
 
     leaving = &so;
-    if (!kFull || phase != kTrackMesh) do {
-      // One step through a voxelized solid (track_through_ggems_voxelized_solid,
-      // TrackThroughGGEMSVoxelizedSolid.cl:133-310) or a detector box
-      // (track_through_ggems_solid_box, TrackThroughGGEMSSolidBox.cl:122-248):
-      // the same sampling and slab test against the current voxel or the whole
-      // box (material 0), then each solid's own tail.
+    const uint32_t pack = static_cast<uint32_t>(n0.y);
+    if (!kFull || phase != kTrackMesh) {
+      // Up to kTrackSteps steps through a voxelized solid
+      // (track_through_ggems_voxelized_solid, TrackThroughGGEMSVoxelizedSolid.cl:133-310)
+      // or a detector box (track_through_ggems_solid_box,
+      // TrackThroughGGEMSSolidBox.cl:122-248): the same sampling and slab test
+      // against the current voxel or the whole box (a grid of one voxel of
+      // material 0), then each solid's own tail.  A step that neither leaves the
+      // solid nor interacts nor falls below a cut has no branch between the
+      // voxel index and its end, so that the label's load, the three draws and
+      // the slab test overlap; everything else is behind one test.
       const bool voxel = phase == kTrackVoxel;
-      V3 vmin = bmin, vmax = bmax;
-      int material = 0;
-      if (voxel) {
-        V3 vs = v3(s1.z, s1.w, s2.x);
-        V3 q = sub(ph.p, bmin);
-        q = s4.w ? mul(q, v3(s2.y, s2.z, s2.w)) : divv(q, vs);
-        int ix = __float2int_rz(q.x), iy = __float2int_rz(q.y), iz = __float2int_rz(q.z);
+      const float threshold = voxel ? 0.0f : so.threshold;
+      const float* cuts = reinterpret_cast<const float*>(tab.base + static_cast<uint32_t>(n0.w));
+#pragma unroll 1
+      for (int k = 0; k < (kDose ? kTrackStepsDose : kTrackSteps); ++k) {
+        const float4 s0 = load4f(&so.border_min[0]);     // border_min xyz, border_max x
+        const float4 s1 = load4f(&so.border_max[1]);     // border_max yz, voxel_sizes xy
+        const float4 s2 = load4f(&so.voxel_sizes[2]);    // voxel_sizes z, inv_voxel_sizes xyz
+        const int4 s4 = load4i(&so.labels);              // labels (2 words)
+        const V3 bmin = v3(s0.x, s0.y, s0.z), bmax = v3(s0.w, s1.x, s1.y), vs = v3(s1.z, s1.w, s2.x);
         const int nx = s3.x, ny = s3.y, nz = s3.z;
-        if (ix >= nx || iy >= ny || iz >= nz || ix < 0 || iy < 0 || iz < 0) {
+        V3 q = sub(ph.p, bmin);
+        int ix, iy, iz;
+        V3 vmin, vmax;
+        bool outside;
+        if (P.voxel_mode != kVoxelGeneral) {
+          q = P.voxel_mode == kVoxelPow2 ? mul(q, v3(s2.y, s2.z, s2.w))
+                                         : v3(quotient(q.x, vs.x, s2.y), quotient(q.y, vs.y, s2.z), quotient(q.z, vs.z, s2.w));
+          // trunc(q) without the conversion pipe: 2^23 + q rounded towards
+          // zero holds trunc(q) in its low bits (and a q of 2^23 or more gives
+          // bits beyond any n); a q in (-1, 0) truncates to voxel 0, one of
+          // -1 or less is outside
+          const float mx = __fadd_rz(fmaxf(q.x, 0.0f), kTwo23), my = __fadd_rz(fmaxf(q.y, 0.0f), kTwo23),
+                      mz = __fadd_rz(fmaxf(q.z, 0.0f), kTwo23);
+          vmin = add(bmin, mul(v3(mx - kTwo23, my - kTwo23, mz - kTwo23), vs));
+          vmax = add(vmin, vs);
+          ix = __float_as_int(mx) - __float_as_int(kTwo23);
+          iy = __float_as_int(my) - __float_as_int(kTwo23);
+          iz = __float_as_int(mz) - __float_as_int(kTwo23);
+          outside = ix >= nx || iy >= ny || iz >= nz || fminf(fminf(q.x, q.y), q.z) <= -1.0f;
+        } else {
+          q = voxel ? divv(q, vs) : v3(0.0f, 0.0f, 0.0f);
+          ix = __float2int_rz(q.x);
+          iy = __float2int_rz(q.y);
+          iz = __float2int_rz(q.z);
+          outside = ix >= nx || iy >= ny || iz >= nz || ix < 0 || iy < 0 || iz < 0;
+          vmin = add(bmin, mul(v3(static_cast<float>(ix), static_cast<float>(iy), static_cast<float>(iz)), vs));
+          vmax = voxel ? add(vmin, vs) : bmax;
+        }
+        if (outside) {
           ph.psd = kOutOfWorld;
           ph.solid_id = -1;
           leave = 1;
@@ -1297,64 +1367,67 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
         }
         const uint8_t* labels = reinterpret_cast<const uint8_t*>(
             (static_cast<unsigned long long>(static_cast<uint32_t>(s4.y)) << 32) | static_cast<uint32_t>(s4.x));
-        material = __ldg(labels + (ix + iy * nx + iz * nx * ny));
-        vmin = add(bmin, mul(v3(static_cast<float>(ix), static_cast<float>(iy), static_cast<float>(iz)), vs));
-        vmax = add(vmin, vs);
-      }
-      int proc;
-      float nid = next_interaction(rng, n0.x, static_cast<uint32_t>(n0.y), sig, energy_id, material, proc);
-      ph.p = safety_inside(ph.p, vmin, vmax);
-      float dtb = distance_to_aabb(ph.p, ph.d, inv_d, vmin, vmax);
-      if (dtb <= nid) {
-        nid = dtb + kTolerance;
-        proc = GG_TRANSPORTATION;
-        if (kDose && voxel && so.dose_map >= 0) {
+        const int material = __ldg(labels + (ix + iy * nx + iz * nx * ny));
+        int proc;
+        float nid = next_interaction(rng, pack, P.fast_sampling != 0,
+                                     sig + (material * n0.x + energy_id) * row_stride(pack), proc);
+        ph.p = safety_inside(ph.p, vmin, vmax);
+        const float dtb = distance_to_aabb(ph.p, ph.d, inv_d, vmin, vmax);
+        const bool crosses = dtb <= nid;
+        if (kDose && P.photon_tracking && crosses && voxel && so.dose_map >= 0) {
           const DevDoseMap& dm = P.dose_maps[so.dose_map];
           if (dm.photon_tracking) {
             int id = dosel(dm, ph.p);
             if (id >= 0) atomicAdd(dm.photon_tracking + id, 1);
           }
         }
-      }
-      ph.p = safety_outside(add(ph.p, scale(ph.d, nid)), vmin, vmax);
-      if (!in_aabb(ph.p, bmin, bmax)) {
-        ph.psd = kOutOfWorld;
-        ph.solid_id = -1;
-        leave = 1;
-        break;
-      }
-      if (!voxel) {
-        if (ph.E < so.threshold) ph.status = GG_DEAD;
-      } else if (kDose && so.dose_tle) {
-        // The step's deposit depends only on the energy before the interaction,
-        // so it is recorded here even when the interaction itself is deferred.
-        dose_record(P.dose_maps[so.dose_map], tle_edep(tab.attenuation(nav), material, ph.E, nid), ph.p);
-      }
-      trk(GG_TRACK_STEP, ph.solid_id, proc);
-      if (proc == GG_COMPTON_SCATTERING || proc == GG_RAYLEIGH_SCATTERING) {
-        pending = (proc << 8) | material;
-        phase = kInteract;
-        continue;
-      }
-      if (!voxel) {
-        if (proc == GG_PHOTOELECTRIC_EFFECT) {
-          ph.status = GG_DEAD;
-          ph.E = 0.0f;
-          box_histogram(so, ph);
+        nid = crosses ? dtb + kTolerance : nid;
+        proc = crosses ? GG_TRANSPORTATION : proc;
+        ph.p = safety_outside(add(ph.p, scale(ph.d, nid)), vmin, vmax);
+        const bool inside = in_aabb(ph.p, bmin, bmax);
+        const float cut = cuts[material];
+        if (kDose && P.tle && inside && voxel && so.dose_tle) {
+          // The step's deposit depends only on the energy before the interaction,
+          // so it is recorded here even when the interaction itself is deferred.
+          dose_record(P.dose_maps[so.dose_map], tle_edep(tab.attenuation(nav), material, ph.E, nid), ph.p);
         }
-      } else {
-        if (proc == GG_PHOTOELECTRIC_EFFECT) {
-          if (kDose && so.dose_map >= 0 && !so.dose_tle) dose_record(P.dose_maps[so.dose_map], ph.E, ph.p);
-          ph.status = GG_DEAD;
-          ph.E = 0.0f;
+        if (kAux && inside) trk(GG_TRACK_STEP, ph.solid_id, proc);
+        if (inside && proc == GG_TRANSPORTATION && ph.E > cut && ph.E >= threshold) continue;
+        if (!inside) {
+          ph.psd = kOutOfWorld;
+          ph.solid_id = -1;
+          leave = 1;
+          break;
         }
-        if (ph.E <= reinterpret_cast<const float*>(tab.base + static_cast<uint32_t>(n0.w))[material]) {
-          if (kDose && so.dose_map >= 0) dose_record(P.dose_maps[so.dose_map], ph.E, ph.p);
-          ph.status = GG_DEAD;
+        if (!voxel && ph.E < threshold) ph.status = GG_DEAD;
+        if (proc == GG_COMPTON_SCATTERING || proc == GG_RAYLEIGH_SCATTERING) {
+          pending = (proc << 8) | material;
+          phase = kInteract;
+          break;
+        }
+        if (!voxel) {
+          if (proc == GG_PHOTOELECTRIC_EFFECT) {
+            ph.status = GG_DEAD;
+            ph.E = 0.0f;
+            box_histogram(so, ph);
+          }
+        } else {
+          if (proc == GG_PHOTOELECTRIC_EFFECT) {
+            if (kDose && so.dose_map >= 0 && !so.dose_tle) dose_record(P.dose_maps[so.dose_map], ph.E, ph.p);
+            ph.status = GG_DEAD;
+            ph.E = 0.0f;
+          }
+          if (ph.E <= cut) {
+            if (kDose && so.dose_map >= 0) dose_record(P.dose_maps[so.dose_map], ph.E, ph.p);
+            ph.status = GG_DEAD;
+          }
+        }
+        if (ph.status == GG_DEAD) {
+          leave = 2;
+          break;
         }
       }
-      if (ph.status == GG_DEAD) leave = 2;
-    } while (0);
+    }
     else if (kFull && phase == kTrackMesh) do {
       // track_through_ggems_meshed_solid, TrackThroughGGEMSMeshSolid.cl:385-518:
       // the parity of the crossing count says whether the photon is inside the
@@ -1373,7 +1446,7 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
         next = x.second;
       }
       int proc;
-      float nid = next_interaction(rng, n0.x, static_cast<uint32_t>(n0.y), sig, energy_id, 0, proc);
+      float nid = next_interaction(rng, pack, P.fast_sampling != 0, sig + energy_id * row_stride(pack), proc);
       const float dx = next.x - ph.p.x, dy = next.y - ph.p.y, dz = next.z - ph.p.z;
       const float to_next = sqrtf(dx * dx + dy * dy + dz * dz);
       if (to_next <= nid) {
