@@ -227,7 +227,14 @@ cudaError_t set_rayleigh_fit(const float* pp);
 void launch_compute_dose(const DoseParams& p, void* stream);
 
 // Line integrals of mu through a voxelized solid, one ray per detector element
-// (source point -> element centre), for the scatter surrogate's inputs.
+// (source point -> element centre), for the scatter surrogate's inputs: all
+// projections of a call in one launch.
+struct RayFrame {                // one projection
+  float detector_matrix[16];
+  float detector_min[3];
+  float element_size[3];
+  float source[3];               // world
+};
 struct ProjectorParams {
   float phantom_matrix[16];
   float border_min[3], border_max[3];
@@ -236,12 +243,10 @@ struct ProjectorParams {
   const uint8_t* labels;
   const float* mu;               // per material, mm^-1
   int32_t number_of_materials;
-  float detector_matrix[16];
-  float detector_min[3];
-  float element_size[3];
   int32_t elements[2];
-  float source[3];               // world
-  float* out;                    // [elements[1]][elements[0]], or [..][..][2] with network_input
+  int32_t count;                 // projections
+  const RayFrame* frames;        // [count], device
+  float* out;                    // [count][elements[1]][elements[0]], or [..][..][..][2] with network_input
   int32_t network_input;         // 1: write (exp(-L), L) pairs, the surrogate network's input
 };
 void launch_line_integrals(const ProjectorParams& p, void* stream);

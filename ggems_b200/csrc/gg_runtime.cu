@@ -1308,6 +1308,71 @@ int autotune(gg_context* c, const std::function<int()>& trial, float* best_ms) {
 
 }  // namespace
 
+namespace {
+
+// The projector's launch (gg_line_integrals, gg_line_integrals_batch): one
+// upload of the projections' frames, the attenuation and the labels, one
+// kernel for all projections.  Stream-ordered buffers: no device-wide
+// synchronisation (cudaFree would wait for transport running on other streams).
+int project(gg_context* c, const gg_solid* phantom, const gg_solid* detectors, const float* source_positions,
+            int32_t count, const float* mu, int32_t number_of_materials, bool network_input, float* out,
+            bool out_on_device) {
+  GG_CUDA(cudaSetDevice(c->device));
+  gg::ProjectorParams P{};
+  std::memcpy(P.phantom_matrix, phantom->obb.matrix, sizeof(P.phantom_matrix));
+  std::memcpy(P.border_min, phantom->obb.border_min, sizeof(P.border_min));
+  std::memcpy(P.border_max, phantom->obb.border_max, sizeof(P.border_max));
+  std::memcpy(P.number_of_voxels, phantom->number_of_voxels, sizeof(P.number_of_voxels));
+  std::memcpy(P.voxel_sizes, phantom->voxel_sizes, sizeof(P.voxel_sizes));
+  P.number_of_materials = number_of_materials;
+  P.elements[0] = detectors[0].virtual_element_number[0];
+  P.elements[1] = detectors[0].virtual_element_number[1];
+  P.count = count;
+  P.network_input = network_input ? 1 : 0;
+  std::vector<gg::RayFrame> frames(count);
+  for (int k = 0; k < count; ++k) {
+    gg::RayFrame& f = frames[k];
+    const gg_solid& d = detectors[k];
+    std::memcpy(f.detector_matrix, d.obb.matrix, sizeof(f.detector_matrix));
+    std::memcpy(f.detector_min, d.obb.border_min, sizeof(f.detector_min));
+    for (int a = 0; a < 3; ++a) f.element_size[a] = d.box_size[a] / static_cast<float>(d.virtual_element_number[a]);
+    std::memcpy(f.source, source_positions + 3 * static_cast<size_t>(k), sizeof(f.source));
+  }
+  const size_t values = static_cast<size_t>(count) * P.elements[0] * P.elements[1] * (network_input ? 2 : 1);
+  const size_t nv = static_cast<size_t>(phantom->number_of_voxels[0]) * phantom->number_of_voxels[1] * phantom->number_of_voxels[2];
+  // frames, attenuation and labels in one buffer, each 256-byte aligned
+  const auto align256 = [](size_t b) { return (b + 255) & ~static_cast<size_t>(255); };
+  const size_t mu_at = align256(frames.size() * sizeof(gg::RayFrame));
+  const size_t labels_at = mu_at + align256(number_of_materials * sizeof(float));
+  unsigned char* buffer = nullptr;
+  float* host_out = nullptr;  // device copy of a host result
+  cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&buffer), labels_at + nv, c->stream);
+  if (e == cudaSuccess && !out_on_device)
+    e = cudaMallocAsync(reinterpret_cast<void**>(&host_out), values * sizeof(float), c->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(buffer, frames.data(), frames.size() * sizeof(gg::RayFrame), cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(buffer + mu_at, mu, number_of_materials * sizeof(float), cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(buffer + labels_at, phantom->labels, nv, cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess) {
+    P.frames = reinterpret_cast<const gg::RayFrame*>(buffer);
+    P.mu = reinterpret_cast<const float*>(buffer + mu_at);
+    P.labels = buffer + labels_at;
+    P.out = out_on_device ? out : host_out;
+    gg::launch_line_integrals(P, c->stream);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess && !out_on_device)
+    e = cudaMemcpyAsync(out, host_out, values * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
+  if (buffer) cudaFreeAsync(buffer, c->stream);
+  if (host_out) cudaFreeAsync(host_out, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  if (e != cudaSuccess) return fail(GG_ERROR_CUDA, std::string("line integrals: ") + cudaGetErrorString(e));
+  return GG_OK;
+}
+
+}  // namespace
+
 extern "C" {
 
 GG_API int gg_autotune(gg_context* c, const gg_source* source, uint64_t number_of_particles, float* best_ms) {
@@ -1331,45 +1396,7 @@ GG_API int gg_line_integrals(gg_context* c, const gg_solid* phantom, const gg_so
   for (int a = 0; a < 3; ++a)
     if (phantom->number_of_voxels[a] < 1 || !(phantom->voxel_sizes[a] > 0.0f) || detector->virtual_element_number[a] < 1)
       return fail(GG_ERROR_INVALID_ARGUMENT, "bad phantom or detector dimensions");
-  GG_CUDA(cudaSetDevice(c->device));
-  gg::ProjectorParams P{};
-  std::memcpy(P.phantom_matrix, phantom->obb.matrix, sizeof(P.phantom_matrix));
-  std::memcpy(P.border_min, phantom->obb.border_min, sizeof(P.border_min));
-  std::memcpy(P.border_max, phantom->obb.border_max, sizeof(P.border_max));
-  std::memcpy(P.number_of_voxels, phantom->number_of_voxels, sizeof(P.number_of_voxels));
-  std::memcpy(P.voxel_sizes, phantom->voxel_sizes, sizeof(P.voxel_sizes));
-  P.number_of_materials = number_of_materials;
-  std::memcpy(P.detector_matrix, detector->obb.matrix, sizeof(P.detector_matrix));
-  std::memcpy(P.detector_min, detector->obb.border_min, sizeof(P.detector_min));
-  for (int a = 0; a < 3; ++a) P.element_size[a] = detector->box_size[a] / static_cast<float>(detector->virtual_element_number[a]);
-  P.elements[0] = detector->virtual_element_number[0];
-  P.elements[1] = detector->virtual_element_number[1];
-  std::memcpy(P.source, source_position, sizeof(P.source));
-  const size_t n = static_cast<size_t>(P.elements[0]) * P.elements[1];
-  const size_t nv = static_cast<size_t>(phantom->number_of_voxels[0]) * phantom->number_of_voxels[1] * phantom->number_of_voxels[2];
-  // stream-ordered buffers (no device-wide synchronisation)
-  float *dmu = nullptr, *dout = nullptr;
-  uint8_t* dlab = nullptr;
-  cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&dmu), number_of_materials * sizeof(float), c->stream);
-  if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void**>(&dlab), nv, c->stream);
-  if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void**>(&dout), n * sizeof(float), c->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(dmu, mu, number_of_materials * sizeof(float), cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dlab, phantom->labels, nv, cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) {
-    P.mu = dmu;
-    P.labels = dlab;
-    P.out = dout;
-    gg::launch_line_integrals(P, c->stream);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess) e = cudaMemcpyAsync(line_integrals, dout, n * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
-  if (dmu) cudaFreeAsync(dmu, c->stream);
-  if (dlab) cudaFreeAsync(dlab, c->stream);
-  if (dout) cudaFreeAsync(dout, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) return fail(GG_ERROR_CUDA, std::string("line integrals: ") + cudaGetErrorString(e));
-  return GG_OK;
+  return project(c, phantom, detector, source_position, 1, mu, number_of_materials, false, line_integrals, false);
 }
 
 GG_API int gg_line_integrals_batch(gg_context* c, const gg_solid* phantom, const gg_solid* detectors,
@@ -1387,59 +1414,13 @@ GG_API int gg_line_integrals_batch(gg_context* c, const gg_solid* phantom, const
     if (detectors[k].type != GG_SOLID_BOX || detectors[k].virtual_element_number[0] != ex ||
         detectors[k].virtual_element_number[1] != ey || ex < 1 || ey < 1)
       return fail(GG_ERROR_INVALID_ARGUMENT, "detectors must be boxes with the same element grid");
+  // `inputs` in this device's memory: the kernel writes it directly
   GG_CUDA(cudaSetDevice(c->device));
-  const size_t n = static_cast<size_t>(ex) * ey;
-  const size_t nv = static_cast<size_t>(phantom->number_of_voxels[0]) * phantom->number_of_voxels[1] * phantom->number_of_voxels[2];
-  // `inputs` in this device's memory: the kernels write it directly
   cudaPointerAttributes pa{};
   const bool on_device = cudaPointerGetAttributes(&pa, inputs) == cudaSuccess &&
                          (pa.type == cudaMemoryTypeDevice || pa.type == cudaMemoryTypeManaged) && pa.device == c->device;
   cudaGetLastError();  // a host pointer unknown to CUDA is not an error here
-  // stream-ordered buffers: no device-wide synchronisation (cudaFree would wait
-  // for transport running on other streams)
-  float *dmu = nullptr, *dout = nullptr;
-  uint8_t* dlab = nullptr;
-  cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&dmu), number_of_materials * sizeof(float), c->stream);
-  if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void**>(&dlab), nv, c->stream);
-  if (e == cudaSuccess && !on_device)
-    e = cudaMallocAsync(reinterpret_cast<void**>(&dout), 2 * n * count * sizeof(float), c->stream);
-  float* const target = on_device ? inputs : dout;
-  auto cleanup = [&]() {
-    if (dmu) cudaFreeAsync(dmu, c->stream);
-    if (dlab) cudaFreeAsync(dlab, c->stream);
-    if (dout) cudaFreeAsync(dout, c->stream);
-  };
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(dmu, mu, number_of_materials * sizeof(float), cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dlab, phantom->labels, nv, cudaMemcpyHostToDevice, c->stream);
-  for (int k = 0; k < count && e == cudaSuccess; ++k) {
-    gg::ProjectorParams P{};
-    std::memcpy(P.phantom_matrix, phantom->obb.matrix, sizeof(P.phantom_matrix));
-    std::memcpy(P.border_min, phantom->obb.border_min, sizeof(P.border_min));
-    std::memcpy(P.border_max, phantom->obb.border_max, sizeof(P.border_max));
-    std::memcpy(P.number_of_voxels, phantom->number_of_voxels, sizeof(P.number_of_voxels));
-    std::memcpy(P.voxel_sizes, phantom->voxel_sizes, sizeof(P.voxel_sizes));
-    P.number_of_materials = number_of_materials;
-    const gg_solid& d = detectors[k];
-    std::memcpy(P.detector_matrix, d.obb.matrix, sizeof(P.detector_matrix));
-    std::memcpy(P.detector_min, d.obb.border_min, sizeof(P.detector_min));
-    for (int a = 0; a < 3; ++a) P.element_size[a] = d.box_size[a] / static_cast<float>(d.virtual_element_number[a]);
-    P.elements[0] = ex;
-    P.elements[1] = ey;
-    std::memcpy(P.source, source_positions + 3 * k, sizeof(P.source));
-    P.mu = dmu;
-    P.labels = dlab;
-    P.out = target + 2 * n * k;
-    P.network_input = 1;
-    gg::launch_line_integrals(P, c->stream);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess && !on_device)
-    e = cudaMemcpyAsync(inputs, dout, 2 * n * count * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
-  cleanup();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) return fail(GG_ERROR_CUDA, std::string("line integrals: ") + cudaGetErrorString(e));
-  return GG_OK;
+  return project(c, phantom, detectors, source_positions, count, mu, number_of_materials, true, inputs, on_device);
 }
 
 GG_API int gg_set_tracking(gg_context* c, int32_t slot, int32_t capacity) {

@@ -1567,84 +1567,129 @@ namespace {
 // centre of detector element (i, j), in the phantom's frame: sum of
 // mu[label] x chord length.  Element centres follow the detector histogram's
 // binning (element (i, j) covers [bmin + i es, bmin + (i+1) es) in x, y).
-__global__ void line_integral_kernel(ProjectorParams P) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
+//
+// One launch walks every projection of a call (blockIdx.z), a block 32 x 8
+// elements, a warp 8 x 4 of them (neighbouring rays read the same label lines).
+// The walk's position does not depend on the labels, so kRayBatch steps are
+// taken at a time: their labels load together, then the chords are summed in
+// order.  What bounds it is the walk's instructions (~100 steps a ray); the
+// label volume stays in L2.  360 projections of 256^2 rays through 64^3 labels:
+// 12.0 ms as one launch each (one dependent label load a step, few rays in
+// flight), 2.9 ms now; 8 projections of 333^2 1.32x.
+constexpr int kRayBatch = 4;
+constexpr int kRayThreads = 256;
+__global__ void __launch_bounds__(kRayThreads) line_integral_kernel(const __grid_constant__ ProjectorParams P) {
+  __shared__ float mu[257];  // by label; 256: a step past the ray's end
+  for (int k = threadIdx.x; k < 257; k += kRayThreads) mu[k] = k < P.number_of_materials && k < 256 ? P.mu[k] : 0.0f;
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * 32 + (warp & 3) * 8 + (lane & 7), j = blockIdx.y * 8 + (warp >> 2) * 4 + (lane >> 3);
   if (i >= P.elements[0] || j >= P.elements[1]) return;
-  const V3 local_pixel = v3(P.detector_min[0] + (static_cast<float>(i) + 0.5f) * P.element_size[0],
-                            P.detector_min[1] + (static_cast<float>(j) + 0.5f) * P.element_size[1], 0.0f);
-  const V3 pixel = l2g_pos(P.detector_matrix, local_pixel);
-  const V3 s = g2l_pos(P.phantom_matrix, v3(P.source[0], P.source[1], P.source[2]));
-  const V3 e = g2l_pos(P.phantom_matrix, pixel);
-  const float dv[3] = {e.x - s.x, e.y - s.y, e.z - s.z};
-  const float sv[3] = {s.x, s.y, s.z};
-  float t0 = 0.0f, t1 = 1.0f;
-  for (int a = 0; a < 3; ++a) {
-    if (fabsf(dv[a]) < 1e-12f) {
-      if (sv[a] < P.border_min[a] || sv[a] > P.border_max[a]) t1 = -1.0f;
-    } else {
-      float ta = (P.border_min[a] - sv[a]) / dv[a], tb = (P.border_max[a] - sv[a]) / dv[a];
-      if (ta > tb) {
-        float t = ta;
-        ta = tb;
-        tb = t;
-      }
-      t0 = fmaxf(t0, ta);
-      t1 = fminf(t1, tb);
-    }
-  }
-  float sum = 0.0f;
-  if (t1 > t0) {
-    const float length = sqrtf(dv[0] * dv[0] + dv[1] * dv[1] + dv[2] * dv[2]);
-    int idx[3], step[3];
-    float tmax[3], tdelta[3];
-    const float tm = 0.5f * (t0 + t1);
+  for (int proj = blockIdx.z; proj < P.count; proj += gridDim.z) {
+    const RayFrame& R = P.frames[proj];
+    const V3 local_pixel = v3(R.detector_min[0] + (static_cast<float>(i) + 0.5f) * R.element_size[0],
+                              R.detector_min[1] + (static_cast<float>(j) + 0.5f) * R.element_size[1], 0.0f);
+    const V3 pixel = l2g_pos(R.detector_matrix, local_pixel);
+    const V3 s = g2l_pos(P.phantom_matrix, v3(R.source[0], R.source[1], R.source[2]));
+    const V3 e = g2l_pos(P.phantom_matrix, pixel);
+    const float dv[3] = {e.x - s.x, e.y - s.y, e.z - s.z};
+    const float sv[3] = {s.x, s.y, s.z};
+    float t0 = 0.0f, t1 = 1.0f;
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
-      // start voxel: the one containing the entry point (nudged inside)
-      const float pa = sv[a] + fminf(t0 + 1e-6f * (t1 - t0), tm) * dv[a];
-      int k = static_cast<int>(floorf((pa - P.border_min[a]) / P.voxel_sizes[a]));
-      idx[a] = min(max(k, 0), P.number_of_voxels[a] - 1);
-      if (dv[a] > 0.0f) {
-        step[a] = 1;
-        tmax[a] = (P.border_min[a] + (idx[a] + 1) * P.voxel_sizes[a] - sv[a]) / dv[a];
-        tdelta[a] = P.voxel_sizes[a] / dv[a];
-      } else if (dv[a] < 0.0f) {
-        step[a] = -1;
-        tmax[a] = (P.border_min[a] + idx[a] * P.voxel_sizes[a] - sv[a]) / dv[a];
-        tdelta[a] = -P.voxel_sizes[a] / dv[a];
+      if (fabsf(dv[a]) < 1e-12f) {
+        if (sv[a] < P.border_min[a] || sv[a] > P.border_max[a]) t1 = -1.0f;
       } else {
-        step[a] = 0;
-        tmax[a] = FLT_MAX;
-        tdelta[a] = FLT_MAX;
+        float ta = (P.border_min[a] - sv[a]) / dv[a], tb = (P.border_max[a] - sv[a]) / dv[a];
+        if (ta > tb) {
+          float t = ta;
+          ta = tb;
+          tb = t;
+        }
+        t0 = fmaxf(t0, ta);
+        t1 = fminf(t1, tb);
       }
     }
-    float t = t0;
-    const int nx = P.number_of_voxels[0], nxy = nx * P.number_of_voxels[1];
-    for (int guard = 0; guard < 4 * (P.number_of_voxels[0] + P.number_of_voxels[1] + P.number_of_voxels[2]); ++guard) {
-      const int a = (tmax[0] < tmax[1]) ? (tmax[0] < tmax[2] ? 0 : 2) : (tmax[1] < tmax[2] ? 1 : 2);
-      const float tn = fminf(tmax[a], t1);
-      const int m = P.labels[idx[0] + idx[1] * nx + idx[2] * nxy];
-      if (m < P.number_of_materials) sum += P.mu[m] * (tn - t) * length;
-      t = tn;
-      if (t >= t1) break;
-      idx[a] += step[a];
-      if (idx[a] < 0 || idx[a] >= P.number_of_voxels[a]) break;
-      tmax[a] += tdelta[a];
+    float sum = 0.0f;
+    if (t1 > t0) {
+      const float length = sqrtf(dv[0] * dv[0] + dv[1] * dv[1] + dv[2] * dv[2]);
+      int left[3], stride[3];  // voxels ahead on the axis; label offset of a step
+      float tmax[3], tdelta[3];
+      const float tm = 0.5f * (t0 + t1);
+      int offset = 0;
+      int pitch = 1;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        // start voxel: the one containing the entry point (nudged inside)
+        const float pa = sv[a] + fminf(t0 + 1e-6f * (t1 - t0), tm) * dv[a];
+        int k = static_cast<int>(floorf((pa - P.border_min[a]) / P.voxel_sizes[a]));
+        k = min(max(k, 0), P.number_of_voxels[a] - 1);
+        offset += k * pitch;
+        if (dv[a] > 0.0f) {
+          left[a] = P.number_of_voxels[a] - 1 - k;
+          stride[a] = pitch;
+          tmax[a] = (P.border_min[a] + (k + 1) * P.voxel_sizes[a] - sv[a]) / dv[a];
+          tdelta[a] = P.voxel_sizes[a] / dv[a];
+        } else if (dv[a] < 0.0f) {
+          left[a] = k;
+          stride[a] = -pitch;
+          tmax[a] = (P.border_min[a] + k * P.voxel_sizes[a] - sv[a]) / dv[a];
+          tdelta[a] = -P.voxel_sizes[a] / dv[a];
+        } else {
+          left[a] = 0x7fffffff;
+          stride[a] = 0;
+          tmax[a] = FLT_MAX;
+          tdelta[a] = FLT_MAX;
+        }
+        pitch *= P.number_of_voxels[a];
+      }
+      float t = t0;
+      bool on = true;
+      int guard = 4 * (P.number_of_voxels[0] + P.number_of_voxels[1] + P.number_of_voxels[2]);
+      while (on) {
+        int label[kRayBatch];
+        float chord[kRayBatch];
+#pragma unroll
+        for (int k = 0; k < kRayBatch; ++k) {
+          const bool x_first = tmax[0] < tmax[1];
+          const bool z_next = !((x_first ? tmax[0] : tmax[1]) < tmax[2]);
+          const bool ax = x_first && !z_next, ay = !x_first && !z_next;
+          const float tn = fminf(z_next ? tmax[2] : (ax ? tmax[0] : tmax[1]), t1);
+          label[k] = on ? static_cast<int>(__ldg(P.labels + offset)) : 256;
+          chord[k] = tn - t;
+          t = tn;
+          const int ahead = z_next ? left[2] : (ax ? left[0] : left[1]);
+          on = on && !(t >= t1) && ahead > 0 && --guard > 0;
+          offset += on ? (z_next ? stride[2] : (ax ? stride[0] : stride[1])) : 0;
+          left[0] -= ax ? 1 : 0;
+          left[1] -= ay ? 1 : 0;
+          left[2] -= z_next ? 1 : 0;
+          tmax[0] = ax ? tmax[0] + tdelta[0] : tmax[0];
+          tmax[1] = ay ? tmax[1] + tdelta[1] : tmax[1];
+          tmax[2] = z_next ? tmax[2] + tdelta[2] : tmax[2];
+        }
+#pragma unroll
+        for (int k = 0; k < kRayBatch; ++k) {
+          const float add = mu[label[k]] * chord[k] * length;
+          sum = label[k] < 256 ? sum + add : sum;
+        }
+      }
     }
-  }
-  const size_t o = static_cast<size_t>(j) * P.elements[0] + i;
-  if (P.network_input) {
-    P.out[2 * o] = expf(-sum);
-    P.out[2 * o + 1] = sum;
-  } else {
-    P.out[o] = sum;
+    const size_t o = (static_cast<size_t>(proj) * P.elements[1] + j) * P.elements[0] + i;
+    if (P.network_input) {
+      P.out[2 * o] = expf(-sum);
+      P.out[2 * o + 1] = sum;
+    } else {
+      P.out[o] = sum;
+    }
   }
 }
 
 }  // namespace
 
 void launch_line_integrals(const ProjectorParams& p, void* stream) {
-  dim3 grid((p.elements[0] + 127) / 128, p.elements[1]);
-  line_integral_kernel<<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  dim3 grid((p.elements[0] + 31) / 32, (p.elements[1] + 7) / 8, p.count < 65535 ? p.count : 65535);
+  line_integral_kernel<<<grid, kRayThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
 }
 
 void launch_compute_dose(const DoseParams& p, void* stream) {
