@@ -18,6 +18,7 @@
 #include <string>
 #include <vector>
 
+#include "gg_copy.cuh"
 #include "gg_internal.cuh"
 
 namespace {
@@ -114,6 +115,9 @@ struct gg_context {
   float last_ms = 0.0f;
   int64_t last_launches = 0;
   bool scene_ready = false;
+  // where gg_read_tallies converts energies on their way to pageable memory
+  double* tally_scratch = nullptr;
+  size_t tally_scratch_doubles = 0;
 };
 
 namespace {
@@ -183,6 +187,8 @@ void free_scene(gg_context* c, bool keep_buffers = false) {
   c->world_energy = nullptr;
   c->world_energy_squared = nullptr;
   c->world_momentum = nullptr;
+  c->tally_scratch = nullptr;
+  c->tally_scratch_doubles = 0;
   c->scene_ready = false;
 }
 
@@ -501,6 +507,7 @@ GG_API int gg_context_create(int32_t device_index, gg_context** context) {
   if (prop.major < 10) return fail(GG_ERROR_NO_DEVICE, std::string("device is not sm_100 class: ") + prop.name);
   gg_context* c = new gg_context();
   c->device = device_index;
+  gg::hold_staging(device_index);
   c->sm_count = prop.multiProcessorCount;
   c->smem_optin = prop.sharedMemPerBlockOptin;
   if (const char* v = std::getenv("GGEMS_B200_REGROUP_LANES")) {
@@ -576,6 +583,7 @@ GG_API int gg_context_destroy(gg_context* c) {
   if (c->start) cudaEventDestroy(c->start);
   if (c->stop) cudaEventDestroy(c->stop);
   if (c->stream) cudaStreamDestroy(c->stream);
+  gg::release_staging(c->device);
   delete c;
   return GG_OK;
 }
@@ -601,10 +609,12 @@ GG_API int gg_set_random_states(gg_context* c, const uint32_t* states, int64_t n
     return fail(GG_ERROR_INVALID_ARGUMENT, "bad random state arguments");
   GG_CUDA(cudaSetDevice(c->device));
   const size_t S = GG_MAXIMUM_PARTICLES;
+  if (number_of_slots == GG_MAXIMUM_PARTICLES) {  // the five arrays are one
+    GG_CUDA(gg::copy_to_device(c->device, c->stream, c->rng, states, 5 * S * sizeof(uint32_t)));
+    return GG_OK;
+  }
   for (int k = 0; k < 5; ++k)
-    GG_CUDA(cudaMemcpyAsync(c->rng + k * S, states + k * S, number_of_slots * sizeof(uint32_t), cudaMemcpyHostToDevice,
-                            c->stream));
-  GG_CUDA(cudaStreamSynchronize(c->stream));
+    GG_CUDA(gg::copy_to_device(c->device, c->stream, c->rng + k * S, states + k * S, number_of_slots * sizeof(uint32_t)));
   return GG_OK;
 }
 
@@ -613,10 +623,10 @@ GG_API int gg_get_random_states(gg_context* c, uint32_t* states, int64_t number_
     return fail(GG_ERROR_INVALID_ARGUMENT, "bad random state arguments");
   GG_CUDA(cudaSetDevice(c->device));
   const size_t S = GG_MAXIMUM_PARTICLES;
+  gg::HostCopy copies[5];
   for (int k = 0; k < 5; ++k)
-    GG_CUDA(cudaMemcpyAsync(states + k * S, c->rng + k * S, number_of_slots * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                            c->stream));
-  GG_CUDA(cudaStreamSynchronize(c->stream));
+    copies[k] = gg::HostCopy{states + k * S, c->rng + k * S, number_of_slots * sizeof(uint32_t), false};
+  GG_CUDA(gg::copies_to_host(c->device, c->stream, copies, 5));
   return GG_OK;
 }
 
@@ -786,6 +796,13 @@ GG_API int gg_upload_scene(gg_context* c, const gg_scene* sc) {
     if (w.energy_squared_tracking && (rc = dev_copy<double>(c, nullptr, cells, &c->world_energy_squared))) return rc;
     if (w.momentum && (rc = dev_copy<unsigned long long>(c, nullptr, 3 * cells, &c->world_momentum))) return rc;
   }
+
+  c->tally_scratch_doubles = c->world_energy || c->world_momentum ? c->world_cells : 0;
+  for (const gg::DevDoseMap& m : c->dose_host)
+    c->tally_scratch_doubles = std::max(c->tally_scratch_doubles, static_cast<size_t>(m.total_number_of_dosels));
+  // larger arrays are converted on the staged path
+  c->tally_scratch_doubles = std::min(c->tally_scratch_doubles, gg::kStagedCopyBytes / 8);
+  if ((rc = dev_copy<double>(c, nullptr, c->tally_scratch_doubles, &c->tally_scratch))) return rc;
 
   // ---- solids ----
   std::vector<gg::DevSolid> solids(sc->number_of_solids);
@@ -1468,70 +1485,59 @@ GG_API int gg_last_run_stats(gg_context* c, float* milliseconds, int64_t* kernel
 
 }  // extern "C"
 
-namespace {
-// n int64 fixed-point tallies (LSB 2^-32 MeV) into the caller's doubles: the
-// integers land in the caller's array itself (same size), whose page-locked
-// memory the copy then uses if it is, and are converted in place.
-cudaError_t read_fixed_point(double* dst, const unsigned long long* src, size_t n) {
-  cudaError_t e = cudaMemcpy(dst, src, n * 8, cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return e;
-  long long* q = reinterpret_cast<long long*>(dst);
-  for (size_t i = 0; i < n; ++i) {
-    long long v;
-    std::memcpy(&v, q + i, sizeof(v));
-    dst[i] = static_cast<double>(v) / gg::kEdepScale;
-  }
-  return cudaSuccess;
-}
-}  // namespace
-
 extern "C" {
 
 GG_API int gg_read_tallies(gg_context* c, gg_tally_buffers* t) {
   if (!c || !t) return fail(GG_ERROR_INVALID_ARGUMENT, "NULL argument");
   if (!c->scene_ready) return fail(GG_ERROR_STATE, "no scene uploaded");
   GG_CUDA(cudaSetDevice(c->device));
-  GG_CUDA(cudaStreamSynchronize(c->stream));
+  // work that another library queued on the default stream (a collective on the
+  // device tallies) comes first
+  GG_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+  // every requested array in one set of copies; energies (int64 fixed point)
+  // become doubles on the way
+  std::vector<gg::HostCopy> copies;
+  auto add = [&](void* host, const void* device, size_t bytes, bool fixed_point) {
+    if (host && device) copies.push_back(gg::HostCopy{host, device, bytes, fixed_point});
+  };
   for (size_t h = 0; h < c->histograms.size(); ++h)
-    if (t->histograms && t->histograms[h])
-      GG_CUDA(cudaMemcpy(t->histograms[h], c->histograms[h], c->histogram_sizes[h] * 4, cudaMemcpyDeviceToHost));
+    if (t->histograms) add(t->histograms[h], c->histograms[h], static_cast<size_t>(c->histogram_sizes[h]) * 4, false);
   for (size_t d = 0; d < c->dose_host.size(); ++d) {
     const gg::DevDoseMap& m = c->dose_host[d];
     const size_t n = static_cast<size_t>(m.total_number_of_dosels);
-    if (t->edep && t->edep[d]) GG_CUDA(read_fixed_point(t->edep[d], m.edep, n));
-    if (t->edep_squared && t->edep_squared[d] && m.edep_squared)
-      GG_CUDA(cudaMemcpy(t->edep_squared[d], m.edep_squared, n * 8, cudaMemcpyDeviceToHost));
-    if (t->hit && t->hit[d] && m.hit) GG_CUDA(cudaMemcpy(t->hit[d], m.hit, n * 4, cudaMemcpyDeviceToHost));
-    if (t->photon_tracking && t->photon_tracking[d] && m.photon_tracking)
-      GG_CUDA(cudaMemcpy(t->photon_tracking[d], m.photon_tracking, n * 4, cudaMemcpyDeviceToHost));
+    if (t->edep) add(t->edep[d], m.edep, n * 8, true);
+    if (t->edep_squared) add(t->edep_squared[d], m.edep_squared, n * 8, false);
+    if (t->hit) add(t->hit[d], m.hit, n * 4, false);
+    if (t->photon_tracking) add(t->photon_tracking[d], m.photon_tracking, n * 4, false);
   }
   const size_t w = c->world_cells;
-  auto read_fixed = [&](double* dst, const unsigned long long* src) { return read_fixed_point(dst, src, w); };
-  if (t->world_photon_tracking && c->world_photon)
-    GG_CUDA(cudaMemcpy(t->world_photon_tracking, c->world_photon, w * 4, cudaMemcpyDeviceToHost));
-  if (t->world_energy && c->world_energy) GG_CUDA(read_fixed(t->world_energy, c->world_energy));
-  if (t->world_energy_squared && c->world_energy_squared)
-    GG_CUDA(cudaMemcpy(t->world_energy_squared, c->world_energy_squared, w * 8, cudaMemcpyDeviceToHost));
+  add(t->world_photon_tracking, c->world_photon, w * 4, false);
+  add(t->world_energy, c->world_energy, w * 8, true);
+  add(t->world_energy_squared, c->world_energy_squared, w * 8, false);
   if (c->world_momentum) {
     double* m[3] = {t->world_momentum_x, t->world_momentum_y, t->world_momentum_z};
-    for (int a = 0; a < 3; ++a)
-      if (m[a]) GG_CUDA(read_fixed(m[a], c->world_momentum + a * w));
+    for (int a = 0; a < 3; ++a) add(m[a], c->world_momentum + a * w, w * 8, true);
   }
+  GG_CUDA(gg::copies_to_host(c->device, c->stream, copies.data(), static_cast<int>(copies.size()), c->tally_scratch,
+                             c->tally_scratch_doubles * 8));
   return GG_OK;
 }
 
 GG_API int gg_read_particles(gg_context* c, gg_particle_buffers* b, int64_t n) {
   if (!c || !b || n < 0 || n > GG_MAXIMUM_PARTICLES) return fail(GG_ERROR_INVALID_ARGUMENT, "bad arguments");
   GG_CUDA(cudaSetDevice(c->device));
-  GG_CUDA(cudaStreamSynchronize(c->stream));
+  GG_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
   const gg::DevParticles& p = c->particles;
-  float* dst[7] = {b->E, b->px, b->py, b->pz, b->dx, b->dy, b->dz};
-  float* src[7] = {p.E, p.px, p.py, p.pz, p.dx, p.dy, p.dz};
-  for (int k = 0; k < 7; ++k)
-    if (dst[k]) GG_CUDA(cudaMemcpy(dst[k], src[k], n * 4, cudaMemcpyDeviceToHost));
-  if (b->status) GG_CUDA(cudaMemcpy(b->status, p.status, n, cudaMemcpyDeviceToHost));
-  if (b->scatter) GG_CUDA(cudaMemcpy(b->scatter, p.scatter, n, cudaMemcpyDeviceToHost));
-  if (b->solid_id) GG_CUDA(cudaMemcpy(b->solid_id, p.solid_id, n * 4, cudaMemcpyDeviceToHost));
+  const size_t m = static_cast<size_t>(n);
+  const gg::HostCopy all[10] = {{b->E, p.E, m * 4, false},   {b->px, p.px, m * 4, false}, {b->py, p.py, m * 4, false},
+                                {b->pz, p.pz, m * 4, false}, {b->dx, p.dx, m * 4, false}, {b->dy, p.dy, m * 4, false},
+                                {b->dz, p.dz, m * 4, false}, {b->status, p.status, m, false},
+                                {b->scatter, p.scatter, m, false}, {b->solid_id, p.solid_id, m * 4, false}};
+  gg::HostCopy copies[10];
+  int count = 0;
+  for (const gg::HostCopy& k : all)
+    if (k.host) copies[count++] = k;
+  GG_CUDA(gg::copies_to_host(c->device, c->stream, copies, count));
   return GG_OK;
 }
 
@@ -1568,9 +1574,8 @@ GG_API int gg_compute_dose(gg_context* c, int32_t dose_map, int32_t solid, float
   P.uncertainty = uncertainty ? c->dose_out + n : nullptr;
   gg::launch_compute_dose(P, c->stream);
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dose, P.dose, n * 4, cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess && uncertainty) e = cudaMemcpyAsync(uncertainty, P.uncertainty, n * 4, cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  const gg::HostCopy copies[2] = {{dose, P.dose, n * 4, false}, {uncertainty, P.uncertainty, n * 4, false}};
+  if (e == cudaSuccess) e = gg::copies_to_host(c->device, c->stream, copies, uncertainty ? 2 : 1);
   if (e != cudaSuccess) return fail(GG_ERROR_CUDA, std::string("compute dose: ") + cudaGetErrorString(e));
   return GG_OK;
 }

@@ -44,6 +44,7 @@
 #include <vector>
 
 #include "ggems_b200.h"
+#include "gg_copy.cuh"
 #include "gg_unet_umma.cuh"
 
 namespace {
@@ -433,6 +434,7 @@ int grid_for(size_t n) { return static_cast<int>(std::min<size_t>((n + 255) / 25
 // ------------------------------------------------------------------ network --
 struct gg_unet {
   int batch = 0, size = 0;
+  int device = 0;
   cudaStream_t stream = nullptr;
   struct Layer {
     int cin, cout, side;  // input / output channels, spatial side
@@ -600,6 +602,8 @@ GG_API int gg_unet_create(int32_t batch, int32_t size, uint64_t seed, gg_unet** 
   gg_unet* n = new gg_unet();
   n->batch = batch;
   n->size = size;
+  if (cudaGetDevice(&n->device) != cudaSuccess) n->device = 0;
+  gg::hold_staging(n->device);
   auto drop = [&](int rc) {
     gg_unet_destroy(n);
     return rc;
@@ -685,6 +689,7 @@ GG_API int gg_unet_destroy(gg_unet* n) {
   for (void* p : n->allocations) cudaFree(p);
   if (n->conv_error_host) cudaFreeHost(n->conv_error_host);
   if (n->stream) cudaStreamDestroy(n->stream);
+  gg::release_staging(n->device);
   delete n;
   return GG_OK;
 }
@@ -693,14 +698,14 @@ GG_API int64_t gg_unet_parameter_count(const gg_unet* n) { return n ? static_cas
 
 GG_API int gg_unet_get_parameters(gg_unet* n, float* host) {
   if (!n || !host) return unet_fail(GG_ERROR_INVALID_ARGUMENT, "NULL argument");
-  UNET_CUDA(cudaMemcpyAsync(host, n->params, n->n_params * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
-  UNET_CUDA(cudaStreamSynchronize(n->stream));
+  const gg::HostCopy copy{host, n->params, n->n_params * sizeof(float), false};
+  UNET_CUDA(gg::copies_to_host(n->device, n->stream, &copy, 1));
   return GG_OK;
 }
 
 GG_API int gg_unet_set_parameters(gg_unet* n, const float* host) {
   if (!n || !host) return unet_fail(GG_ERROR_INVALID_ARGUMENT, "NULL argument");
-  UNET_CUDA(cudaMemcpyAsync(n->params, host, n->n_params * sizeof(float), cudaMemcpyHostToDevice, n->stream));
+  UNET_CUDA(gg::copy_to_device(n->device, n->stream, n->params, host, n->n_params * sizeof(float)));
   int rc;
   if ((rc = refresh_weights(n))) return rc;
   UNET_CUDA(cudaStreamSynchronize(n->stream));
@@ -725,9 +730,11 @@ GG_API int gg_unet_gradients(gg_unet* n, const float* input, const float* target
   int rc;
   if ((rc = forward(n, input)) || (rc = backward(n, target))) return rc;
   if (loss) UNET_CUDA(cudaMemcpyAsync(loss, n->loss, sizeof(float), cudaMemcpyDeviceToHost, n->stream));
-  if (grads_host)
-    UNET_CUDA(cudaMemcpyAsync(grads_host, n->grads, n->n_params * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
   if ((rc = queue_conv_status(n))) return rc;
+  if (grads_host) {
+    const gg::HostCopy copy{grads_host, n->grads, n->n_params * sizeof(float), false};
+    UNET_CUDA(gg::copies_to_host(n->device, n->stream, &copy, 1));
+  }
   UNET_CUDA(cudaStreamSynchronize(n->stream));
   return conv_status(n);
 }

@@ -19,6 +19,7 @@
 #include <string>
 #include <type_traits>
 
+#include "gg_copy.cuh"
 #include "gg_internal.cuh"
 
 struct gg_volume {
@@ -328,6 +329,7 @@ GG_API int gg_volume_create(int32_t device_index, int32_t met_type, const int32_
   VOL_CUDA(cudaSetDevice(device_index));
   gg_volume* v = new gg_volume();
   v->device = device_index;
+  gg::hold_staging(device_index);
   v->met_type = met_type;
   std::memcpy(v->dimensions, dimensions, sizeof(v->dimensions));
   std::memcpy(v->element_sizes, element_sizes, sizeof(v->element_sizes));
@@ -359,6 +361,7 @@ GG_API int gg_volume_destroy(gg_volume* v) {
   if (v->start) cudaEventDestroy(v->start);
   if (v->stop) cudaEventDestroy(v->stop);
   if (v->stream) cudaStreamDestroy(v->stream);
+  gg::release_staging(v->device);
   delete v;
   return GG_OK;
 }
@@ -367,8 +370,7 @@ GG_API int gg_volume_upload(gg_volume* v, const void* host, uint64_t bytes) {
   if (!v || !host) return gg::record_error(GG_ERROR_INVALID_ARGUMENT, "NULL argument");
   if (bytes != v->elements * v->element_bytes) return gg::record_error(GG_ERROR_INVALID_ARGUMENT, "image size mismatch");
   VOL_CUDA(cudaSetDevice(v->device));
-  VOL_CUDA(cudaMemcpyAsync(v->data, host, bytes, cudaMemcpyHostToDevice, v->stream));
-  VOL_CUDA(cudaStreamSynchronize(v->stream));
+  VOL_CUDA(gg::copy_to_device(v->device, v->stream, v->data, host, bytes));
   return GG_OK;
 }
 
@@ -376,8 +378,8 @@ GG_API int gg_volume_download(gg_volume* v, void* host, uint64_t bytes) {
   if (!v || !host) return gg::record_error(GG_ERROR_INVALID_ARGUMENT, "NULL argument");
   if (bytes != v->elements * v->element_bytes) return gg::record_error(GG_ERROR_INVALID_ARGUMENT, "image size mismatch");
   VOL_CUDA(cudaSetDevice(v->device));
-  VOL_CUDA(cudaMemcpyAsync(host, v->data, bytes, cudaMemcpyDeviceToHost, v->stream));
-  VOL_CUDA(cudaStreamSynchronize(v->stream));
+  const gg::HostCopy copy{host, v->data, static_cast<size_t>(bytes), false};
+  VOL_CUDA(gg::copies_to_host(v->device, v->stream, &copy, 1));
   return GG_OK;
 }
 
@@ -443,9 +445,9 @@ GG_API int gg_volume_labels(gg_volume* v, const float* range_first, const float*
   VOL_CUDA(cudaGetLastError());
   VOL_CUDA(cudaEventRecord(v->stop, v->stream));
   unsigned long long m = 0;
-  VOL_CUDA(cudaMemcpyAsync(labels, v->labels, v->elements, cudaMemcpyDeviceToHost, v->stream));
-  VOL_CUDA(cudaMemcpyAsync(&m, v->missing, sizeof(m), cudaMemcpyDeviceToHost, v->stream));
-  VOL_CUDA(cudaStreamSynchronize(v->stream));
+  const gg::HostCopy copies[2] = {{labels, v->labels, static_cast<size_t>(v->elements), false},
+                                  {&m, v->missing, sizeof(m), false}};
+  VOL_CUDA(gg::copies_to_host(v->device, v->stream, copies, 2));
   VOL_CUDA(cudaEventElapsedTime(&v->last_ms, v->start, v->stop));
   if (unconverted) *unconverted = static_cast<int64_t>(m);
   return GG_OK;

@@ -1,0 +1,82 @@
+"""Host copies through the page-locked slots: sizes at the edges of the staged
+path and of a slot, unaligned host addresses, page-locked arrays, several threads
+at once (more than there are staging blocks), and the energies' conversion on the
+way (on the device for maps below the staged size, and on the staged path)."""
+
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+
+import parity
+import scenes
+from ggems_b200 import abi
+
+pytestmark = pytest.mark.gpu
+
+STAGED = 48 << 20  # kStagedCopyBytes
+SIZES = [1, 524_289, STAGED - 1, STAGED, STAGED + 1, STAGED + 524_288, 70_000_001]
+
+
+def _round_trip(n, seed, offset=0, pinned=False):
+    from ggems_b200._native import Volume, check, lib
+    rng = np.random.default_rng(seed)
+    src = rng.integers(0, 256, n + offset, dtype=np.uint8)[offset:]
+    if pinned:
+        import torch
+        back = torch.empty(n, dtype=torch.uint8, pin_memory=True).numpy()
+    else:
+        back = np.empty(n + offset, np.uint8)[offset:]
+    v = Volume(abi.GG_MET_UCHAR, (n, 1, 1), (1.0, 1.0, 1.0))
+    check(lib.gg_volume_upload(v.handle, C.c_void_p(src.ctypes.data), n))
+    check(lib.gg_volume_download(v.handle, C.c_void_p(back.ctypes.data), n))
+    v.close()
+    return np.array_equal(src, back)
+
+
+@pytest.mark.parametrize("n", SIZES)
+def test_round_trip(n):
+    assert _round_trip(n, 1)
+    assert _round_trip(n, 2, offset=3)
+
+
+def test_page_locked_and_threads():
+    assert _round_trip(STAGED + 5, 3, pinned=True)
+    ok = [False] * 4
+
+    def work(k):
+        ok[k] = all(_round_trip(STAGED + 777 * k, 10 + k) for _ in range(3))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(ok))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert all(ok)
+
+
+@pytest.mark.parametrize("n", [16, 200])
+def test_energies_are_converted_on_the_way(n):
+    """The int64 tally on the device, divided by 2^32, whatever path the copy takes
+    (200^3 dosels are 64 MB)."""
+    import torch
+    from ggems_b200 import _native
+    from ggems_b200.distributed import device_tallies
+    sc = scenes.water_box_scene(n=n, voxel=128.0 / n)
+    src = scenes.XRaySource(monoenergy=scenes.F(60.0) * scenes.KEV, aperture_deg=6.0)
+    ctx = _native.Context(0)
+    try:
+        _, T, _ = parity.run_gpu(ctx, sc, src, 20000)
+        q = device_tallies(ctx.handle)[0].cpu().numpy()
+        assert q.dtype == np.int64 and q.any()
+        want = q.astype(np.float64) / 4294967296.0
+        assert np.array_equal(T.edep[0], want)
+        # page-locked arrays: written by the device
+        pinned = abi.Tallies([], [n ** 3], alloc=lambda k, t: torch.zeros(
+            k, dtype={np.int32: torch.int32, np.float64: torch.float64}[t], pin_memory=True).numpy())
+        ctx.read_tallies(pinned)
+        assert np.array_equal(pinned.edep[0], want)
+        assert np.array_equal(pinned.hit[0], T.hit[0]) and np.array_equal(pinned.edep_squared[0], T.edep_squared[0])
+    finally:
+        ctx.close()
