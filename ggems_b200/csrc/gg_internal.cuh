@@ -37,9 +37,10 @@ constexpr uint32_t kPackCount = 0x7fu, kPackReciprocals = 0x80u;
 // Voxel index of a solid: general (divisions, integer conversions),
 // multiplication by an exact 2^-k, or quotient() with the correctly rounded
 // reciprocal; the last two for at most 2^22 voxels an axis (trunc by rounding
-// at 2^23).  A box is a grid of one voxel: reciprocal 0, so that every position
-// has index 0.  A launch takes the first of general, reciprocal, pow2 that one
-// of its solids needs.
+// at 2^23) in a grid where the voxel step's short forms hold (fast_steps in
+// gg_runtime.cu).  A launch takes the first of general, reciprocal, pow2 that one
+// of its voxelized solids needs; general: whole steps only.  A box takes whole
+// steps too, as a grid of one voxel.
 constexpr int kVoxelGeneral = 0, kVoxelPow2 = 1, kVoxelReciprocal = 2, kVoxelBox = 3;
 // Tables with reciprocals may take this much of a block's shared memory: three
 // blocks of 256 threads with the photon stash stay resident per SM.  Larger
@@ -81,16 +82,19 @@ struct DevDoseMap {
 };
 
 struct alignas(16) DevSolid {
-  // read by every tracking step: the first 80 bytes, five vector loads
+  // read by every tracking step: the first 88 bytes, vector loads
   float border_min[3];
-  float border_max[3];
   float voxel_sizes[3];
   float inv_voxel_sizes[3];      // 1 / voxel_sizes correctly rounded (exact for powers of two)
+  float inner_min[3];            // border_min + kTolerance, border_max - kTolerance
+  float inner_max[3];
+  uint32_t label_bias;           // bits of 2^23f * (nx ny + nx + 1): the voxel step's label index is that much too large
   int32_t number_of_voxels[3];
   int32_t navigator;
   const uint8_t* labels;
   int32_t type;
   int32_t voxel_mode;            // how the voxel index divides by the voxel size (kVoxel*)
+  float border_max[3];
   float matrix[16];
   float threshold;
   int32_t virtual_element_number[3];
@@ -187,6 +191,7 @@ struct TransportParams {
   int32_t* tracking_count;
   int32_t voxel_mode;               // kVoxelGeneral, kVoxelReciprocal or kVoxelPow2: what serves every solid of the launch
   int32_t fast_sampling;            // every navigator: all three processes, sigma rows with reciprocals
+  int32_t shared_grids;             // batched launch: every job's voxelized solids have the first job's grids
   int32_t photon_tracking;          // some dose map counts photons
   int32_t tle;                      // some dose map uses the track-length estimator
   int32_t regroup_lanes;            // waiting lanes that start a round of the rare phases (1..32)

@@ -404,6 +404,25 @@ int upload_mesh(gg_context* c, const gg_solid& g, gg::DevSolid* d, std::vector<v
 }
 
 
+// Whether the transport kernel's voxel step may take its short forms in this
+// grid: voxels of at least 16 kTolerance, coordinates of at most 2048 mm (then
+// the roundings of a voxel's faces and of a position's index, below 3.1e-4 mm
+// together, stay below kTolerance), and an index within the grid for both ends
+// of the range kTolerance inside the borders, hence for all positions between
+// them (difference and quotient are monotonic).
+bool fast_steps(const gg_solid& g) {
+  constexpr float kTolerance = 5.0e-04f;
+  for (int a = 0; a < 3; ++a) {
+    const float lo = g.obb.border_min[a], hi = g.obb.border_max[a], v = g.voxel_sizes[a];
+    const int n = g.number_of_voxels[a];
+    if (!(v >= 16.0f * kTolerance && static_cast<double>(v) * n <= 2048.0 && lo >= -2048.0f && hi <= 2048.0f)) return false;
+    const volatile float first = (lo + kTolerance) - lo, last = (hi - kTolerance) - lo;
+    const float q0 = first / v, q1 = last / v;
+    if (!(q0 >= 0.0f && q1 >= 0.0f && q1 < static_cast<float>(n))) return false;
+  }
+  return true;
+}
+
 // Device form of one solid; labels and mesh arrays are uploaded into `owner`
 // (once per host array when `labels_seen` is given).
 int make_dev_solid(gg_context* c, const gg_solid& g, gg::DevSolid* out, std::vector<void*>& owner,
@@ -433,17 +452,18 @@ int make_dev_solid(gg_context* c, const gg_solid& g, gg::DevSolid* out, std::vec
     reciprocal &= v >= gg::kQuotientMin && v <= gg::kQuotientMax && g.number_of_voxels[a] <= (1 << 22);
     d.inv_voxel_sizes[a] = 1.0f / v;
   }
-  d.voxel_mode = !reciprocal ? gg::kVoxelGeneral : (pow2 ? gg::kVoxelPow2 : gg::kVoxelReciprocal);
+  d.voxel_mode = !(reciprocal && fast_steps(g)) ? gg::kVoxelGeneral : (pow2 ? gg::kVoxelPow2 : gg::kVoxelReciprocal);
+  constexpr float kTolerance = 5.0e-04f;  // as gg_transport.cu
+  for (int a = 0; a < 3; ++a) {
+    d.inner_min[a] = d.border_min[a] + kTolerance;
+    d.inner_max[a] = d.border_max[a] - kTolerance;
+  }
+  const uint32_t nx = static_cast<uint32_t>(g.number_of_voxels[0]), ny = static_cast<uint32_t>(g.number_of_voxels[1]);
+  d.label_bias = 0x4b000000u * (nx * ny + nx + 1u);
   if (g.type == GG_SOLID_BOX) {
-    // one voxel of material 0, where that reproduces the borders bit for bit
-    bool same = true;
-    for (int a = 0; a < 3; ++a) {
-      d.number_of_voxels[a] = 1;
-      d.voxel_sizes[a] = d.border_max[a] - d.border_min[a];
-      d.inv_voxel_sizes[a] = 0.0f;
-      same &= d.border_min[a] + d.voxel_sizes[a] == d.border_max[a];
-    }
-    d.voxel_mode = same ? gg::kVoxelBox : gg::kVoxelGeneral;
+    // the transport kernel takes it as a grid of one voxel of material 0
+    for (int a = 0; a < 3; ++a) d.number_of_voxels[a] = 1;
+    d.voxel_mode = gg::kVoxelBox;
   }
   std::memcpy(d.virtual_element_number, g.virtual_element_number, sizeof(d.virtual_element_number));
   std::memcpy(d.box_size, g.box_size, sizeof(d.box_size));
@@ -1017,6 +1037,13 @@ int prepare_jobs(gg_context* c, const gg_job* jobs, int32_t n, std::vector<void*
   };
   for (int s = 0; s < c->number_of_solids; ++s) need_mode(c->solid_dev_host[s]);
   for (const gg::DevSolid& d : job_solids) need_mode(d);
+  P.shared_grids = 1;
+  for (size_t i = 0; i < job_solids.size(); ++i) {
+    // everything that the voxel steps read before the labels
+    const gg::DevSolid& first = job_solids[i % c->number_of_solids];
+    if (job_solids[i].type == GG_SOLID_VOXELIZED || first.type == GG_SOLID_VOXELIZED)
+      P.shared_grids &= std::memcmp(&job_solids[i], &first, offsetof(gg::DevSolid, labels)) == 0 ? 1 : 0;
+  }
   P.fast_sampling = 1;
   for (uint32_t pack : c->process_pack) P.fast_sampling &= (pack & 0xffu) == (3u | gg::kPackReciprocals) ? 1 : 0;
   for (const gg::DevDoseMap& m : c->dose_host) P.photon_tracking |= m.photon_tracking ? 1 : 0;

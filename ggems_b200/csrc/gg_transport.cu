@@ -14,9 +14,11 @@
 //    slot's histories in batch order, so every history draws exactly the
 //    random numbers the reference's slot would; lanes fetch slots from a
 //    device work counter;
-//  * a lane advances one "step" per loop iteration (a voxel step, a box step,
-//    or a FindSolid/ProjectToSolid round), and starts its next history as
-//    soon as one ends, so lanes never idle while others finish long histories;
+//  * a lane takes up to kTrackSteps voxel steps that need no logarithm (the
+//    draws show that the photon crosses its voxel), or one part of anything else
+//    (a whole step, an interaction, a FindSolid/ProjectToSolid round) per loop
+//    iteration, and starts its next history as soon as one ends, so lanes never
+//    idle while others finish long histories;
 //  * the per-navigator cross-section tables (float4 per material and energy
 //    bin), energy bins and photon cuts are staged into shared memory with
 //    cp.async.bulk completing on an mbarrier (bounded wait);
@@ -53,16 +55,17 @@ constexpr float kKissTwoToMinus32 = 0x1p-32f;
 constexpr float kKissCorrection = -0x1.ffp-56f;  // -(2^-23 - 2^-32) * 2^-32, exact in float
 
 // Tracking steps a lane takes between two looks at its warp's waiting photons.
-// The look (ballots, counts, the stash's exchange test) costs every lane about
-// as much as a fifth of a step; a lane that stops early idles for the rest.
-// Without dose maps 1 / 2 / 4 / 8 steps: CBCT 33.4 / 32.0 / 30.4 / 29.9 ms per
-// 1e7 primaries, 36 projections of 1e6 31.6 / 30.3 / 28.0 / 26.5 ms.  With dose
-// maps the steps diverge at their tallies: C1 water 1.20 ms at 2 and 1.22 to
-// 1.23 at 1 and 3, TLE emission 11.2 at 2, 11.7 and 12.1.
-constexpr int kTrackSteps = 8, kTrackStepsDose = 2;
+// The look (ballots, counts, the stash's exchange test) costs every lane more
+// than a step; a lane that stops early idles for the rest.  5 / 8 / 12 / 20
+// steps: CBCT of 1e8 primaries 177 / 172 / 166 / 165 ms, 36 projections of 1e6
+// 27.6 / 26.9 / 26.4 / 26.3 ms, 64^3 dose of 1e6 1.84 / 1.81 / 1.83 / 1.76 ms.
+constexpr int kTrackSteps = 16;
 constexpr float kTwo23 = 8388608.0f;
 
-enum Phase : int { kNewHistory = 0, kFind = 1, kTrackVoxel = 2, kTrackBox = 3, kTrackMesh = 4, kInteract = 5, kDone = 6 };
+// kTrackVoxel: steps of a voxelized solid that surely cross their voxel.
+// kInteract: any other step of a voxelized solid, any step of a detector box, or
+// the Compton / Rayleigh part of a meshed solid's step.
+enum Phase : int { kNewHistory = 0, kFind = 1, kTrackVoxel = 2, kTrackMesh = 4, kInteract = 5, kDone = 6 };
 
 struct V3 {
   float x, y, z;
@@ -112,6 +115,7 @@ __device__ __forceinline__ V3 rotate_uz(V3 v, V3 u) {
 // BinarySearch / LinearInterpolation, GGEMSMathAlgorithms.hh:46-86
 __device__ __forceinline__ int binary_search(float key, const float* a, int size) {
   int low = 0, high = size - 1;
+#pragma unroll 1
   while (high - low > 1) {
     int mid = (high + low) / 2;
     float v = a[mid];
@@ -189,15 +193,20 @@ __device__ __forceinline__ float distance_to_aabb(V3 p, V3 d, V3 inv, V3 mn, V3 
   return miss ? kOutOfWorld : t;
 }
 
-__device__ __forceinline__ V3 reciprocal(V3 d) { return v3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z); }
+// Along a face (|d| < 1e-6) the reciprocal is infinite: distance_to_aabb does
+// not read it there, and in the voxel step a face so far away never is the nearest.
+__device__ __forceinline__ float reciprocal(float d) { return fabsf(d) < kEps6 ? __int_as_float(0x7f800000) : 1.0f / d; }
+__device__ __forceinline__ V3 reciprocal(V3 d) { return v3(reciprocal(d.x), reciprocal(d.y), reciprocal(d.z)); }
 __device__ __forceinline__ float distance_to_aabb(V3 p, V3 d, V3 mn, V3 mx) {
   return distance_to_aabb(p, d, reciprocal(d), mn, mx);
 }
 
 // JKISS32, GGEMSKissEngine.hh:50-75
+__device__ __forceinline__ float kiss_uniform(float x) { return __fmaf_rn(x, kKissCorrection, x * kKissTwoToMinus32); }
 struct Kiss {
   uint32_t s1, s2, s3, s4, s5;
-  __device__ __forceinline__ float uniform() {
+  // the draw as a float in [0, 2^32]
+  __device__ __forceinline__ float raw() {
     s2 ^= (s2 << 5);
     s2 ^= (s2 >> 7);
     s2 ^= (s2 << 22);
@@ -206,9 +215,9 @@ struct Kiss {
     s5 = t < 0;
     s4 = static_cast<uint32_t>(t) & 2147483647u;
     s1 += 1411392427u;
-    const float x = __uint2float_rn(s1 + s2 + s4);
-    return __fmaf_rn(x, kKissCorrection, x * kKissTwoToMinus32);
+    return __uint2float_rn(s1 + s2 + s4);
   }
+  __device__ __forceinline__ float uniform() { return kiss_uniform(raw()); }
 };
 
 struct Photon {
@@ -255,45 +264,56 @@ __device__ __forceinline__ float quotient(float a, float b, float y) {
   return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
 }
 
-// GetPhotonNextInteraction, GGEMSPhotonNavigator.hh:57-93.  Returns the
-// distance, writes the process; `row` is the sigma table's row of the material
-// and the cached BinarySearch result (process order; two float4 with the
-// reciprocals in the second when process_pack says so), process_pack the
-// navigator's process count and ids (DevNavigator).  fast: every navigator of
-// the launch has all three processes and reciprocals; then the three draws,
-// logarithms and quotients have no branch and overlap.  A cross section of 0
-// gives NaN there, which is not below nid, as the reference's infinite distance
-// is not.
-__device__ __forceinline__ float next_interaction(Kiss& rng, uint32_t process_pack, bool fast, const float4* row,
-                                                  int& proc) {
-  float nid = kOutOfWorld;
-  const float4 s = row[0];
+// The draws of one GetPhotonNextInteraction call before their conversion to
+// (0, 1): one per process, in process order (0 where a process is missing).
+struct Draws {
+  float x0, x1, x2;
+};
+__device__ __forceinline__ Draws draw_processes(Kiss& rng, uint32_t process_pack, bool fast) {
+  Draws w{0.0f, 0.0f, 0.0f};
   if (fast) {
-    const float4 y = row[1];
-    const float a0 = -logf(rng.uniform()), a1 = -logf(rng.uniform()), a2 = -logf(rng.uniform());
-    const float d0 = quotient(a0, s.x, y.x), d1 = quotient(a1, s.y, y.y), d2 = quotient(a2, s.z, y.z);
-    int shift = 0;
-    if (d0 < nid) {
-      nid = d0;
-      shift = 8;
-    }
-    if (d1 < nid) {
-      nid = d1;
-      shift = 16;
-    }
-    if (d2 < nid) {
-      nid = d2;
-      shift = 24;
-    }
-    proc = shift == 0 ? kNoProcess : static_cast<int>((process_pack >> shift) & 0xffu);
-    return nid;
+    w.x0 = rng.raw();
+    w.x1 = rng.raw();
+    w.x2 = rng.raw();
+    return w;
   }
+  const int n = static_cast<int>(process_pack & kPackCount);
+  if (n > 0) w.x0 = rng.raw();
+  if (n > 1) w.x1 = rng.raw();
+  if (n > 2) w.x2 = rng.raw();
+  return w;
+}
+
+// True only if every process's sampled distance -logf(u) / sigma is at least
+// `distance`, which most steps show without a logarithm or a division: with
+// x = the draw of u (u <= x / 2^32), -log(u) >= 1 - u >= 1 - x / 2^32, so
+// sigma distance + x / 2^32 < 1 is enough.  The scale's 2^-18 covers the
+// roundings of the product (2^-23), of logf (1 ulp, taken as 2^-22) and of the
+// quotient (2^-24); the limit's 2^11 those of the sum (at most 2^8).  False
+// where the test cannot tell (an infinite or NaN product among them); about the
+// share of the steps that interact (1 - u against -log(u): half a per cent more
+// of them at sigma distance = 0.01).
+constexpr float kCrossScale = 0x1.00004p+32f;
+constexpr float kCrossLimit = 0x1p+32f - 0x1p+11f;
+__device__ __forceinline__ bool surely_crosses(Draws w, float4 sigma, float distance) {
+  const float reach = distance * kCrossScale;
+  return __fmaf_rn(sigma.x, reach, w.x0) < kCrossLimit && __fmaf_rn(sigma.y, reach, w.x1) < kCrossLimit &&
+         __fmaf_rn(sigma.z, reach, w.x2) < kCrossLimit;
+}
+
+// GetPhotonNextInteraction, GGEMSPhotonNavigator.hh:57-93, of these draws.
+// Returns the distance, writes the process; sigma is the table's row of the
+// material and the cached BinarySearch result (process order), process_pack the
+// navigator's process count and ids (DevNavigator).  One logarithm and one
+// division in a loop: it runs for few steps, and its code for many warps' sake
+// has to be short (see the kernel's comment on its instruction footprint).
+__device__ __forceinline__ float next_interaction(Draws w, uint32_t process_pack, float4 sigma, int& proc) {
+  float nid = kOutOfWorld;
   proc = kNoProcess;
   const int n = static_cast<int>(process_pack & kPackCount);
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    if (i >= n) break;
-    const float dist = -logf(rng.uniform()) / pick(s, i);
+#pragma unroll 1
+  for (int i = 0; i < n; ++i) {
+    const float dist = -logf(kiss_uniform(i == 0 ? w.x0 : (i == 1 ? w.x1 : w.x2))) / pick(sigma, i);
     if (dist < nid) {
       nid = dist;
       proc = static_cast<int>((process_pack >> (8 * (i + 1))) & 0xffu);
@@ -308,22 +328,25 @@ __device__ __forceinline__ int row_stride(uint32_t process_pack) { return (proce
 __device__ __forceinline__ float4 load4f(const void* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ int4 load4i(const void* p) { return *reinterpret_cast<const int4*>(p); }
 
-// State handed to and returned by the (out-of-line) interaction samplers.
-// Passed by value so that the photon and its random state stay in registers
-// in the transport loop (a reference would force them into local memory).
+// State handed to and returned by the (out-of-line) interaction samplers: the
+// photon's energy and the polar angle.  Passed by value so that the photon and
+// its random state stay in registers in the transport loop (a reference would
+// force them into local memory).  What both samplers end with, the azimuth and
+// the rotation into the photon's frame, is in scatter(), once for both: lanes of
+// either kind run it together and its code is there once.
 struct Interaction {
   float E;
-  V3 d;
+  float cost, sint;
   Kiss rng;
-  int dead;
+  int outcome;
 };
+enum : int { kTurned = 0, kUnchanged = 1, kAbsorbed = 2 };
 
 // KleinNishinaComptonSampleSecondaries, GGEMSComptonScatteringModels.hh:47-132
 __device__ __noinline__ Interaction compton(Interaction in) {
   Kiss rng = in.rng;
   float E0 = in.E;
   float E0m = E0 / kElectronMassC2;
-  V3 gd = in.d;
   float eps0 = 1.0f / (1.0f + 2.0f * E0m);
   float eps0sq = eps0 * eps0;
   float alpha1 = -logf(eps0);
@@ -334,6 +357,7 @@ __device__ __noinline__ Interaction compton(Interaction in) {
     ++nloop;
     if (nloop > 1000) {
       in.rng = rng;
+      in.outcome = kUnchanged;
       return in;
     }
     float r1 = rng.uniform();
@@ -351,22 +375,19 @@ __device__ __noinline__ Interaction compton(Interaction in) {
     greject = 1.0f - eps * sint2 / (1.0f + epssq);
   } while (greject < r3);
   if (sint2 < 0.0f) sint2 = 0.0f;
-  float cost = 1.0f - onecost;
-  float sint = sqrtf(sint2);
-  float phi = rng.uniform() * kTwoPi;
-  V3 g = v3(sint * cosf(phi), sint * sinf(phi), cost);
-  g = normalize3(rotate_uz(g, gd));
   in.E = E0 * eps;
-  in.d = g;
+  in.cost = 1.0f - onecost;
+  in.sint = sqrtf(sint2);
   in.rng = rng;
   return in;
 }
 
 __constant__ float c_rayleigh_pp[9][101];
 
-__device__ __forceinline__ float rayleigh_w(float x, float n) {
+__device__ __noinline__ float exp_minus_n_log(float n, float v) { return expf(-n * logf(v)); }
+__device__ __noinline__ float rayleigh_w(float x, float n) {
   return (x < 0.02f) ? n * x * (1.0f - 0.5f * (n - 1.0f) * x * (1.0f - (n - 2.0f) * x / 3.0f))
-                     : 1.0f - expf(-n * logf(1.0f + x));
+                     : 1.0f - exp_minus_n_log(n, 1.0f + x);
 }
 
 // LivermoreRayleighSampleSecondaries, GGEMSRayleighScatteringModels.hh:169-316
@@ -374,11 +395,10 @@ __device__ __noinline__ Interaction rayleigh(Interaction in, const DevNavigator&
                                              const float4* sig, int material, int energy_id) {
   float E0 = in.E;
   if (E0 <= 250.0e-6f) {
-    in.dead = 1;
+    in.outcome = kAbsorbed;
     return in;
   }
   Kiss rng = in.rng;
-  V3 gd = in.d;
   const int nb = nv.number_of_bins;
   int n_minus_one = static_cast<int8_t>(nv.number_of_elements[material] - 1);
   int mixture = nv.element_offset[material];
@@ -390,6 +410,7 @@ __device__ __noinline__ Interaction rayleigh(Interaction in, const DevNavigator&
     float kcs = lerp_ref(ebins[energy_id], pick(row[0], slot), ebins[energy_id + 1], pick(row[stride], slot), E0);
     float x = rng.uniform() * kcs;
     float cs = 0.0f;
+#pragma unroll 1
     for (int i = 0; i < n_minus_one; ++i) {
       int zi = nv.atomic_number[mixture + i];
       const float* pa = nv.rayleigh_per_atom + nb * zi;
@@ -425,13 +446,11 @@ __device__ __noinline__ Interaction rayleigh(Interaction in, const DevNavigator&
     n = 1.0f / n;
     float y = rng.uniform() * w;
     if (y < 0.02f) x = y * n * (1.0f + 0.5f * (n + 1.0f) * y * (1.0f - (n + 2.0f) * y / 3.0f));
-    else x = expf(-n * logf(1.0f - y)) - 1.0f;
+    else x = exp_minus_n_log(n, 1.0f - y) - 1.0f;
     cost = 1.0f - x / (b * xx);
   } while (2.0f * rng.uniform() > 1.0f + cost * cost || cost < -1.0f);
-  float phi = kTwoPi * rng.uniform();
-  float sint = sqrtf((1.0f - cost) * (1.0f + cost));
-  V3 g = v3(sint * cosf(phi), sint * sinf(phi), cost);
-  in.d = normalize3(rotate_uz(g, gd));
+  in.cost = cost;
+  in.sint = sqrtf((1.0f - cost) * (1.0f + cost));
   in.rng = rng;
   return in;
 }
@@ -439,12 +458,17 @@ __device__ __noinline__ Interaction rayleigh(Interaction in, const DevNavigator&
 // Compton or Rayleigh interaction of the photon (proc is one of the two).
 __device__ __forceinline__ void scatter(Photon& ph, Kiss& rng, int proc, const DevNavigator& nv, const float* ebins,
                                         const float4* sig, int material, int energy_id) {
-  Interaction in{ph.E, ph.d, rng, 0};
+  Interaction in{ph.E, 0.0f, 0.0f, rng, kTurned};
   in = proc == GG_COMPTON_SCATTERING ? compton(in) : rayleigh(in, nv, ebins, sig, material, energy_id);
   ph.E = in.E;
-  ph.d = in.d;
   rng = in.rng;
-  if (in.dead) ph.status = GG_DEAD;
+  if (in.outcome == kTurned) {
+    const float phi = rng.uniform() * kTwoPi;
+    float sin_phi, cos_phi;
+    sincosf(phi, &sin_phi, &cos_phi);  // the same bits as sinf and cosf
+    ph.d = normalize3(rotate_uz(v3(in.sint * cos_phi, in.sint * sin_phi, in.cost), ph.d));
+  }
+  if (in.outcome == kAbsorbed) ph.status = GG_DEAD;
 }
 
 // dose_record_standard / dose_photon_tracking, GGEMSDoseRecording.hh:65-118
@@ -469,75 +493,10 @@ __device__ __forceinline__ void dose_record(const DevDoseMap& dm, float edep, V3
   if (dm.edep_squared) atomicAdd(dm.edep_squared + id, static_cast<double>(edep) * static_cast<double>(edep));
 }
 
-// get_primaries_ggems_xray_source, GetPrimariesGGEMSXRaySource.cl:52-143
-__device__ void xray_primary(Photon& ph, Kiss& rng, const DevSource& s, double new_aperture) {
-  double phi = rng.uniform();
-  double theta = rng.uniform();
-  phi *= static_cast<double>(kTwoPi);
-  theta = acos(1.0 - new_aperture * theta);
-  double st = sin(theta);
-  V3 rot = v3(static_cast<float>(cos(phi) * st), static_cast<float>(sin(phi) * st), static_cast<float>(cos(theta)));
-  V3 gp = l2g_pos(s.matrix, v3(0.0f, 0.0f, 0.0f));
-  V3 dir = normalize3(sub(v3(0.0f, 0.0f, 0.0f), gp));
-  dir = normalize3(rotate_uz(rot, dir));
-  gp.x = s.focal_spot_size[0] * (rng.uniform() - 0.5f);
-  gp.y = s.focal_spot_size[1] * (rng.uniform() - 0.5f);
-  gp.z = s.focal_spot_size[2] * (rng.uniform() - 0.5f);
-  gp = l2g_pos(s.matrix, gp);
-  int index = 0;
-  float rnd = 0.0f;
-  if (s.number_of_energy_bins != 1) {
-    rnd = rng.uniform();
-    index = binary_search(rnd, s.energy_cdf, s.number_of_energy_bins + 1);
-  }
-  ph.E = !s.is_interp ? s.energy_spectrum[index]
-                      : lerp_ref(s.energy_cdf[index], s.energy_spectrum[index], s.energy_cdf[index + 1],
-                                 s.energy_spectrum[index + 1], rnd);
-  ph.p = gp;
-  ph.d = dir;
-}
-
-// get_primaries_ggems_voxelized_source, GetPrimariesGGEMSVoxelizedSource.cl:57-150
-__device__ void voxelized_primary(Photon& ph, Kiss& rng, const DevSource& s) {
-  double phi = rng.uniform();
-  double theta = rng.uniform();
-  phi *= static_cast<double>(kTwoPi);
-  theta = acos(1.0 - 2.0 * theta);
-  double st = sin(theta);
-  V3 dir = v3(static_cast<float>(cos(phi) * st), static_cast<float>(sin(phi) * st), static_cast<float>(cos(theta)));
-  float rnd_act = rng.uniform();
-  int ia = binary_search(rnd_act, s.activity_cdf, s.number_of_activity_bins);
-  int vox = s.activity_index[ia];
-  int nx = s.number_of_voxels[0], slice = nx * s.number_of_voxels[1];
-  int iz = vox / slice;
-  int ix = (vox - iz * slice) % nx;
-  int iy = (vox - iz * slice) / nx;
-  V3 bmin = v3(s.border_min[0], s.border_min[1], s.border_min[2]);
-  V3 vs = v3(s.voxel_sizes[0], s.voxel_sizes[1], s.voxel_sizes[2]);
-  V3 vmin = add(bmin, mul(v3(static_cast<float>(ix), static_cast<float>(iy), static_cast<float>(iz)), vs));
-  V3 vmax = add(vmin, vs);
-  V3 p;
-  p.x = bmin.x + (static_cast<float>(ix) + rng.uniform()) * vs.x;
-  p.y = bmin.y + (static_cast<float>(iy) + rng.uniform()) * vs.y;
-  p.z = bmin.z + (static_cast<float>(iz) + rng.uniform()) * vs.z;
-  p = safety_inside(p, vmin, vmax);
-  ph.p = l2g_pos(s.matrix, p);
-  int index = 0;
-  float rnd = 0.0f;
-  if (s.number_of_energy_bins != 1) {
-    rnd = rng.uniform();
-    index = binary_search(rnd, s.energy_cdf, s.number_of_energy_bins + 1);
-  }
-  ph.E = !s.is_interp ? s.energy_spectrum[index]
-                      : lerp_ref(s.energy_cdf[index], s.energy_spectrum[index], s.energy_cdf[index + 1],
-                                 s.energy_spectrum[index + 1], rnd);
-  ph.d = dir;
-}
-
-// Track-length-estimator deposit of one voxel step
-// (TrackThroughGGEMSVoxelizedSolid.cl:286-301): E * mu_en(E, material) * step
-// (mm -> cm), with mu_en interpolated in the 220-bin attenuation table.
-// A new primary out of line (it runs once per history, in the warp's rare
+// A new primary, get_primaries_ggems_xray_source (GetPrimariesGGEMSXRaySource.cl:52-143)
+// or get_primaries_ggems_voxelized_source (GetPrimariesGGEMSVoxelizedSource.cl:57-150):
+// both start with the cone angles and end with the energy, so one copy of that
+// code serves both.  Out of line (it runs once per history, in the warp's rare
 // round): keeps its FP64 cone sampling out of the tracking loop's
 // instruction footprint; state in and out by value, so nothing goes to the
 // stack.  Measured +0.8 % on the CBCT projection.
@@ -547,12 +506,57 @@ struct PrimaryOut {
   Kiss rng;
 };
 __device__ __noinline__ PrimaryOut new_primary(Kiss rng, const DevSource& s) {
-  Photon ph{};
-  if (s.type == GG_SOURCE_XRAY) xray_primary(ph, rng, s, s.new_aperture);
-  else voxelized_primary(ph, rng, s);
-  return PrimaryOut{ph.p, ph.d, ph.E, rng};
+  PrimaryOut out;
+  const bool xray = s.type == GG_SOURCE_XRAY;
+  double phi = rng.uniform();
+  double theta = rng.uniform();
+  phi *= static_cast<double>(kTwoPi);
+  theta = acos(1.0 - (xray ? s.new_aperture : 2.0) * theta);
+  double st, ct, sp, cp;  // sincos gives the same bits as sin and cos
+  sincos(theta, &st, &ct);
+  sincos(phi, &sp, &cp);
+  const V3 rot = v3(static_cast<float>(cp * st), static_cast<float>(sp * st), static_cast<float>(ct));
+  V3 p;
+  if (xray) {
+    p = l2g_pos(s.matrix, v3(0.0f, 0.0f, 0.0f));
+    const V3 dir = normalize3(sub(v3(0.0f, 0.0f, 0.0f), p));
+    out.d = normalize3(rotate_uz(rot, dir));
+    p.x = s.focal_spot_size[0] * (rng.uniform() - 0.5f);
+    p.y = s.focal_spot_size[1] * (rng.uniform() - 0.5f);
+    p.z = s.focal_spot_size[2] * (rng.uniform() - 0.5f);
+  } else {
+    out.d = rot;
+    const float rnd_act = rng.uniform();
+    const int ia = binary_search(rnd_act, s.activity_cdf, s.number_of_activity_bins);
+    const int vox = s.activity_index[ia];
+    const int nx = s.number_of_voxels[0], slice = nx * s.number_of_voxels[1];
+    const int iz = vox / slice, in_slice = vox - iz * slice;
+    const int iy = in_slice / nx, ix = in_slice - iy * nx;
+    const V3 bmin = v3(s.border_min[0], s.border_min[1], s.border_min[2]);
+    const V3 vs = v3(s.voxel_sizes[0], s.voxel_sizes[1], s.voxel_sizes[2]);
+    const V3 vmin = add(bmin, mul(v3(static_cast<float>(ix), static_cast<float>(iy), static_cast<float>(iz)), vs));
+    p.x = bmin.x + (static_cast<float>(ix) + rng.uniform()) * vs.x;
+    p.y = bmin.y + (static_cast<float>(iy) + rng.uniform()) * vs.y;
+    p.z = bmin.z + (static_cast<float>(iz) + rng.uniform()) * vs.z;
+    p = safety_inside(p, vmin, add(vmin, vs));
+  }
+  out.p = l2g_pos(s.matrix, p);
+  int index = 0;
+  float rnd = 0.0f;
+  if (s.number_of_energy_bins != 1) {
+    rnd = rng.uniform();
+    index = binary_search(rnd, s.energy_cdf, s.number_of_energy_bins + 1);
+  }
+  out.E = !s.is_interp ? s.energy_spectrum[index]
+                       : lerp_ref(s.energy_cdf[index], s.energy_spectrum[index], s.energy_cdf[index + 1],
+                                  s.energy_spectrum[index + 1], rnd);
+  out.rng = rng;
+  return out;
 }
 
+// Track-length-estimator deposit of one voxel step
+// (TrackThroughGGEMSVoxelizedSolid.cl:286-301): E * mu_en(E, material) * step
+// (mm -> cm), with mu_en interpolated in the 220-bin attenuation table.
 __device__ __forceinline__ float tle_edep(const float* att, int material, float energy, float step) {
   const float* me = att + GG_ATTENUATION_BINS * (1 + material);
   int e_index = binary_search(energy, att, GG_ATTENUATION_BINS);
@@ -763,18 +767,18 @@ __device__ __noinline__ void track_point(gg_track_point* points, int32_t* count,
 
 // Histogram of interaction sites in a CT detector module (the HISTOGRAM part of
 // TrackThroughGGEMSSolidBox.cl:214-236), with the scatter histogram.
-__device__ __forceinline__ void box_histogram(const DevSolid& so, const Photon& ph) {
+__device__ __noinline__ void box_histogram(const DevSolid& so, V3 p, bool scattered) {
   if (!so.histogram) return;
   V3 bmin = v3(so.border_min[0], so.border_min[1], so.border_min[2]);
   V3 es = divv(v3(so.box_size[0], so.box_size[1], so.box_size[2]),
                v3(static_cast<float>(so.virtual_element_number[0]), static_cast<float>(so.virtual_element_number[1]),
                   static_cast<float>(so.virtual_element_number[2])));
-  V3 q = divv(sub(ph.p, bmin), es);
+  V3 q = divv(sub(p, bmin), es);
   int ix = __float2int_rz(q.x), iy = __float2int_rz(q.y);
   if (ix >= 0 && iy >= 0 && ix < so.virtual_element_number[0] && iy < so.virtual_element_number[1]) {
     int idx = ix + iy * so.virtual_element_number[0];
     atomicAdd(so.histogram + idx, 1);
-    if (so.scatter_histogram && ph.scatter == 1) atomicAdd(so.scatter_histogram + idx, 1);
+    if (so.scatter_histogram && scattered) atomicAdd(so.scatter_histogram + idx, 1);
   }
 }
 
@@ -841,6 +845,16 @@ __device__ __forceinline__ StashMask stash_mask(unsigned part, int h) {
 // the block size stays a launch parameter (128, 256 or 512 threads).
 constexpr int transport_registers(int blocks) { return (65536 / (kBlockThreads * blocks)) & ~7; }
 
+// What bounds the kernel: the issue slots while photons cross large grids (CBCT
+// 256^3: 71 % of them busy), and instruction fetches where events are frequent
+// (36 projections through 64^3: 7 of the 17 cycles between two instructions of a
+// warp), since the warps of an SM are in different parts of the code.  So the
+// rare parts are kept short rather than fast: one copy of the exchange, of the
+// exit from a solid and of the azimuth after an interaction, loops that are not
+// unrolled, logarithms and exponentials out of line.  The samplers and the
+// sources went from 50 to 30 KB: CBCT of 1e8 229 -> 205 ms, 36 projections
+// 32.8 -> 28.8 ms, 64^3 dose 2.25 -> 2.09 ms.
+//
 // kFull: the scene has a meshed solid, a world grid or a tracked particle;
 // kAux: the world walk and particle tracking are compiled in.  Scenes without
 // them run variants compiled without that code, so its instructions and
@@ -859,7 +873,7 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
   DevSolid* scene_solids = reinterpret_cast<DevSolid*>(g_smem + (P.tables_in_smem ? P.table_bytes : 0));
   DevNavigator* navs = reinterpret_cast<DevNavigator*>(scene_solids + P.number_of_solids);
   uint64_t* bar = reinterpret_cast<uint64_t*>(navs + P.number_of_navigators);
-  for (int i = threadIdx.x; i < P.number_of_solids; i += blockDim.x) scene_solids[i] = P.solids[i];
+  for (int i = threadIdx.x; i < P.number_of_solids; i += blockDim.x) scene_solids[i] = kBatch ? P.job_solids[i] : P.solids[i];
   for (int i = threadIdx.x; i < P.number_of_navigators; i += blockDim.x) navs[i] = P.navigators[i];
   Tab tab{P.table_blob, navs};
   if (P.tables_in_smem) {
@@ -871,7 +885,10 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
 
   const size_t S = GG_MAXIMUM_PARTICLES;
   // Solids of the lane's current job: the shared-memory copy for a single
-  // run, the job's own array (global memory) in a batched launch.
+  // run, the job's own array (global memory) in a batched launch.  Where all
+  // jobs have the same grids (the angles of a scan), the voxel steps read those
+  // from the shared-memory copy of the first job's: lanes in different jobs then
+  // read one address, not one each (36 projections of 1e6: 24.0 ms before).
   const DevSolid* solids = scene_solids;
   int job = 0;
   const int number_of_jobs = kBatch ? P.number_of_jobs : 1;
@@ -886,7 +903,7 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
   int energy_id = 0;
   float cached_E = -1.0f;
   int cached_nav = -1;
-  int pending = 0;  // deferred interaction: process << 8 | material
+  int pending = 0;  // process of a meshed solid's deferred interaction
   V3 inv_d = v3(0.0f, 0.0f, 0.0f);  // reciprocal(ph.d) while tracking inside a solid
   int history_number = -1;           // particle tracking: histories of the slot so far
   // particle tracking (full variant only): a point of this lane's photon when
@@ -901,6 +918,7 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
   // GGEMS source run; the slot's random stream carries over from run to run).
   // Returns false when the slot takes part in no job from `from` on.
   auto enter_job = [&](int from) -> bool {
+#pragma unroll 1
     for (int j = from; j < number_of_jobs; ++j) {
       const DevJob& J = P.jobs[j];
       const uint32_t h = slot < J.q ? J.nb : (slot < J.q + 1 && J.r > 0 ? static_cast<uint32_t>(J.r) : 0u);
@@ -957,8 +975,11 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
   };
   // End of track_through_*: back to the global frame; the history goes on
   // (FindSolid) unless the photon died.
-  auto leave_solid = [&](const DevSolid& so, bool dead) {
-    if (kFull && so.type == GG_SOLID_MESHED) {
+  // why: 1 alive, 2 dead, 3 the history ends without a solid left.
+  auto leave_solid = [&](const DevSolid* solid, int why) {
+    const DevSolid& so = *solid;
+    if (why == 3) {
+    } else if (kFull && so.type == GG_SOLID_MESHED) {
       // A meshed solid tracks in world coordinates and, on leaving (dead or
       // not), carries the photon to its OBB boundary (TrackThroughGGEMSMeshSolid.cl:521-533).
       V3 mn = v3(so.border_min[0], so.border_min[1], so.border_min[2]);
@@ -970,12 +991,45 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
       ph.p = l2g_pos(so.matrix, ph.p);
       ph.d = l2g_dir(so.matrix, ph.d);
     }
-    trk(dead ? GG_TRACK_DEAD : GG_TRACK_LEAVE, -1, -1);
-    if (dead) end_history();
+    if (why != 3) trk(why == 2 ? GG_TRACK_DEAD : GG_TRACK_LEAVE, -1, -1);
+    if (why >= 2) end_history();
     else phase = kFind;
   };
-  auto track_phase = [](int type) {
-    return type == GG_SOLID_VOXELIZED ? kTrackVoxel : (kFull && type == GG_SOLID_MESHED) ? kTrackMesh : kTrackBox;
+  auto track_phase = [&](int type) {
+    return type == GG_SOLID_VOXELIZED && P.voxel_mode != kVoxelGeneral ? kTrackVoxel
+           : (kFull && type == GG_SOLID_MESHED)                        ? kTrackMesh
+                                                                       : kInteract;
+  };
+
+  // BinarySearch of the photon's energy in navigator nav's bins, kept while both stay.
+  auto find_energy = [&](int nav, int bins) {
+    if (ph.E == cached_E && nav == cached_nav) return;
+    energy_id = binary_search(ph.E, tab.energy_bins(nav), bins);
+    cached_E = ph.E;
+    cached_nav = nav;
+  };
+  // Moves the photon to the end of a step of length nid in a voxelized solid's
+  // voxel or a detector box; whether that is inside the solid.
+  // inner_min, inner_max: the solid's borders kTolerance inside (in_aabb's bounds).
+  auto step_to = [&](const DevSolid& so, bool voxel, int nav, int material, float nid, int proc, V3 vmin, V3 vmax,
+                     V3 inner_min, V3 inner_max) -> bool {
+    if (kDose && P.photon_tracking && proc == GG_TRANSPORTATION && voxel && so.dose_map >= 0) {
+      const DevDoseMap& dm = P.dose_maps[so.dose_map];
+      if (dm.photon_tracking) {
+        int id = dosel(dm, ph.p);
+        if (id >= 0) atomicAdd(dm.photon_tracking + id, 1);
+      }
+    }
+    ph.p = safety_outside(add(ph.p, scale(ph.d, nid)), vmin, vmax);
+    const bool inside = !(ph.p.x < inner_min.x || ph.p.x > inner_max.x || ph.p.y < inner_min.y || ph.p.y > inner_max.y ||
+                          ph.p.z < inner_min.z || ph.p.z > inner_max.z);
+    if (kDose && P.tle && inside && voxel && so.dose_tle) {
+      // The step's deposit depends only on the energy before the interaction,
+      // so it is recorded here even when an interaction follows.
+      dose_record(P.dose_maps[so.dose_map], tle_edep(tab.attenuation(nav), material, ph.E, nid), ph.p);
+    }
+    if (kAux && inside) trk(GG_TRACK_STEP, ph.solid_id, proc);
+    return inside;
   };
 
   // ---- photon stash (kStash) ----
@@ -1136,40 +1190,48 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
   for (;;) {
     bool round = false, serve_interact = false;
     if (kStash) {
-      unsigned active = __ballot_sync(0xffffffffu, phase != kDone);
-      if (active == 0 && (st_ready | st_int | st_find) == 0) break;
-      unsigned waiting = __ballot_sync(0xffffffffu, is_rare(phase));
-      // Lanes waiting for a rare phase, and lanes without a photon, take
-      // ready photons from the stash (once enough of them wait: an exchange
-      // costs the warp two shared-memory accesses per word).
-      const unsigned want = waiting | ~active;
-      if (st_ready != 0 && __popc(want) >= min(swap_lanes, stash_popc(st_ready))) {
-        exchange(want, st_ready);
-        active = __ballot_sync(0xffffffffu, phase != kDone);
-        waiting = __ballot_sync(0xffffffffu, is_rare(phase));
+      // Two looks, with one copy of the exchange code for both.
+      bool finished = false;
+#pragma unroll 1
+      for (int look = 0; look < 2; ++look) {
+        const unsigned active = __ballot_sync(0xffffffffu, phase != kDone);
+        const unsigned waiting = __ballot_sync(0xffffffffu, is_rare(phase));
+        unsigned lanes = 0;
+        StashMask records = 0;
+        if (look == 0) {
+          finished = active == 0 && (st_ready | st_int | st_find) == 0;
+          if (finished) break;
+          // Lanes waiting for a rare phase, and lanes without a photon, take
+          // ready photons from the stash (once enough of them wait: an exchange
+          // costs the warp two shared-memory accesses per word).
+          lanes = waiting | ~active;
+          if (__popc(lanes) >= min(swap_lanes, stash_popc(st_ready))) records = st_ready;
+        } else {
+          // A round of one kind of rare work when a full warp of it is waiting
+          // (lanes and records), or when the waiting lanes are many against the
+          // tracking ones and no ready photon is left to replace them.
+          const unsigned w_int = __ballot_sync(0xffffffffu, phase == kInteract);
+          const int n_int = __popc(w_int) + stash_popc(st_int);
+          const int n_find = __popc(waiting & ~w_int) + stash_popc(st_find);
+          const int n_wait = __popc(waiting), n_track = __popc(active & ~waiting);
+          round = n_int + n_find > 0 &&
+                  (n_int >= 32 || n_find >= 32 || n_int + n_find >= round_photons || n_track == 0 ||
+                   (n_wait > 0 && (n_wait >= regroup || 4 * n_wait >= ratio4 * n_track)));
+          if (round) {
+            serve_interact = n_int >= 32 ? (n_find < 32 || n_int >= n_find) : (n_find < 32 && n_int >= n_find);
+            // gather: lanes without a photon of the served kind take one from the stash
+            lanes = ~(serve_interact ? w_int : (waiting & ~w_int));
+            records = serve_interact ? st_int : st_find;
+          }
+        }
+        if (records != 0 && lanes != 0) exchange(lanes, records);
       }
-      // A round of one kind of rare work when a full warp of it is waiting
-      // (lanes and records), or when the waiting lanes are many against the
-      // tracking ones and no ready photon is left to replace them.
-      const unsigned w_int = __ballot_sync(0xffffffffu, phase == kInteract);
-      const int n_int = __popc(w_int) + stash_popc(st_int);
-      const int n_find = __popc(waiting & ~w_int) + stash_popc(st_find);
-      const int n_wait = __popc(waiting), n_track = __popc(active & ~waiting);
-      round = n_int + n_find > 0 &&
-              (n_int >= 32 || n_find >= 32 || n_int + n_find >= round_photons || n_track == 0 ||
-               (n_wait > 0 && (n_wait >= regroup || 4 * n_wait >= ratio4 * n_track)));
-      if (round) {
-        serve_interact = n_int >= 32 ? (n_find < 32 || n_int >= n_find) : (n_find < 32 && n_int >= n_find);
-        // gather: lanes without a photon of the served kind take one from the stash
-        const unsigned kind_lanes = serve_interact ? w_int : (waiting & ~w_int);
-        const StashMask kind_records = serve_interact ? st_int : st_find;
-        if (kind_records != 0 && kind_lanes != 0xffffffffu) exchange(~kind_lanes, kind_records);
-      }
+      if (finished) break;
     } else {
       const unsigned active = __ballot_sync(0xffffffffu, phase != kDone);
       if (active == 0) break;
       const unsigned tracking =
-          __ballot_sync(0xffffffffu, phase == kTrackVoxel || phase == kTrackBox || (kFull && phase == kTrackMesh));
+          __ballot_sync(0xffffffffu, phase == kTrackVoxel || (kFull && phase == kTrackMesh));
       const int n_other = __popc(active & ~tracking);
       round = n_other > 0 && (n_other >= regroup || 4 * n_other >= ratio4 * __popc(tracking));
       // A round serves one kind of rare work: the interaction samplers, or the
@@ -1179,19 +1241,99 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
       if (round) serve_interact = 2 * __popc(__ballot_sync(0xffffffffu, phase == kInteract)) >= n_other;
     }
     // A step or an interaction that ends the photon's stay in its solid sets
-    // `leave` (1: alive, 2: dead) and `leaving`, and jumps to the one copy of
+    // `leave` (1: alive, 2: dead; 3: no solid left) and `leaving`, and jumps to the one copy of
     // the exit code at the end of the loop body.
     int leave = 0;
     const DevSolid* leaving = nullptr;
     if (round) {
       if ((phase == kInteract) != serve_interact) continue;
       if (phase == kInteract) {
-        // The Compton / Rayleigh part of a tracking step (the tail of
-        // track_through_*): sample the interaction, then tally as the step would.
         const DevSolid& so = solids[ph.solid_id];
         const int nav = so.navigator;
-        const int material = pending & 0xff;
-        const int proc = pending >> 8;
+        leaving = &so;
+        int material = 0, proc = pending;
+        if (!kFull || so.type != GG_SOLID_MESHED) {
+          // A whole step through a voxelized solid
+          // (track_through_ggems_voxelized_solid, TrackThroughGGEMSVoxelizedSolid.cl:133-310)
+          // or a detector box (track_through_ggems_solid_box,
+          // TrackThroughGGEMSSolidBox.cl:122-248): the same sampling and slab test
+          // against the current voxel or the whole box (a grid of one voxel of
+          // material 0), then each solid's own tail.
+          const bool voxel = so.type == GG_SOLID_VOXELIZED;
+          const int4 n0 = load4i(&navs[nav]);
+          find_energy(nav, n0.x);
+          const uint32_t pack = static_cast<uint32_t>(n0.y);
+          const V3 bmin = v3(so.border_min[0], so.border_min[1], so.border_min[2]);
+          const V3 bmax = v3(so.border_max[0], so.border_max[1], so.border_max[2]);
+          const V3 vs = v3(so.voxel_sizes[0], so.voxel_sizes[1], so.voxel_sizes[2]);
+          const int nx = so.number_of_voxels[0], ny = so.number_of_voxels[1], nz = so.number_of_voxels[2];
+          // one step, or up to kTrackSteps where no solid of the launch has fast steps
+#pragma unroll 1
+          for (int k = 1;; ++k) {
+          V3 q = sub(ph.p, bmin);
+          q = voxel ? divv(q, vs) : v3(0.0f, 0.0f, 0.0f);
+          const int ix = __float2int_rz(q.x), iy = __float2int_rz(q.y), iz = __float2int_rz(q.z);
+          if (ix >= nx || iy >= ny || iz >= nz || ix < 0 || iy < 0 || iz < 0) {
+            ph.psd = kOutOfWorld;
+            ph.solid_id = -1;
+            leave = 1;
+            goto exit_solid;
+          }
+          const V3 vmin = add(bmin, mul(v3(static_cast<float>(ix), static_cast<float>(iy), static_cast<float>(iz)), vs));
+          const V3 vmax = voxel ? add(vmin, vs) : bmax;
+          material = __ldg(so.labels + (ix + iy * nx + iz * nx * ny));
+          const float4* row =
+              reinterpret_cast<const float4*>(tab.base + static_cast<uint32_t>(n0.z)) +
+              (material * n0.x + energy_id) * row_stride(pack);
+          const float cut = reinterpret_cast<const float*>(tab.base + static_cast<uint32_t>(n0.w))[material];
+          float nid = next_interaction(draw_processes(rng, pack, P.fast_sampling != 0), pack, row[0], proc);
+          ph.p = safety_inside(ph.p, vmin, vmax);
+          const float dtb = distance_to_aabb(ph.p, ph.d, inv_d, vmin, vmax);
+          if (dtb <= nid) {
+            nid = dtb + kTolerance;
+            proc = GG_TRANSPORTATION;
+          }
+          if (!step_to(so, voxel, nav, material, nid, proc, vmin, vmax,
+                       v3(so.inner_min[0], so.inner_min[1], so.inner_min[2]),
+                       v3(so.inner_max[0], so.inner_max[1], so.inner_max[2]))) {
+            ph.psd = kOutOfWorld;
+            ph.solid_id = -1;
+            leave = 1;
+            goto exit_solid;
+          }
+          if (!voxel && ph.E < so.threshold) ph.status = GG_DEAD;
+          if (proc == GG_COMPTON_SCATTERING || proc == GG_RAYLEIGH_SCATTERING) break;
+          {
+            if (!voxel) {
+              if (proc == GG_PHOTOELECTRIC_EFFECT) {
+                ph.status = GG_DEAD;
+                ph.E = 0.0f;
+                box_histogram(so, ph.p, ph.scatter == 1);
+              }
+            } else {
+              if (proc == GG_PHOTOELECTRIC_EFFECT) {
+                if (kDose && so.dose_map >= 0 && !so.dose_tle) dose_record(P.dose_maps[so.dose_map], ph.E, ph.p);
+                ph.status = GG_DEAD;
+                ph.E = 0.0f;
+              }
+              if (ph.E <= cut) {
+                if (kDose && so.dose_map >= 0) dose_record(P.dose_maps[so.dose_map], ph.E, ph.p);
+                ph.status = GG_DEAD;
+              }
+            }
+            if (ph.status == GG_DEAD) {
+              leave = 2;
+              goto exit_solid;
+            }
+            if (P.voxel_mode == kVoxelGeneral && k < kTrackSteps) continue;
+            phase = track_phase(so.type);
+            goto resume;
+          }
+          }
+        }
+        // The Compton / Rayleigh part of a tracking step (the tail of
+        // track_through_*): sample the interaction, then tally as the step would.
+        {
         float e0 = ph.E;
         scatter(ph, rng, proc, navs[nav], tab.energy_bins(nav), tab.sigma(nav), material, energy_id);
         trk(GG_TRACK_SCATTER, ph.solid_id, proc);
@@ -1205,16 +1347,15 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
             ph.status = GG_DEAD;
           }
         } else if (proc == GG_COMPTON_SCATTERING) {
-          box_histogram(so, ph);
+          box_histogram(so, ph.p, ph.scatter == 1);
         }
         if (ph.status == GG_DEAD) {
           leave = 2;
-          leaving = &so;
           goto exit_solid;
         }
-        inv_d = reciprocal(ph.d);
         phase = track_phase(so.type);
-        continue;
+        }
+        goto resume;
       }
       if (phase == kNewHistory) {
         const DevSource& source = P.jobs[job].source;
@@ -1240,6 +1381,7 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
       } else if (!end) {
         ++rounds;
         // particle_solid_distance_* (ParticleSolidDistanceGGEMS*.cl:43-108)
+#pragma unroll 1
         for (int s = 0; s < P.number_of_solids; ++s) {
           if (ph.status == GG_DEAD || ph.psd == 0.0f) break;
           const DevSolid& so = solids[s];
@@ -1284,146 +1426,103 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
             ph.d = g2l_dir(so.matrix, ph.d);
           }
           trk(GG_TRACK_ENTER, ph.solid_id, -1);
-          inv_d = reciprocal(ph.d);
           phase = track_phase(so.type);
         }
       }
-      if (end) end_history();
-      continue;
+      if (end) {
+        leave = 3;
+        goto exit_solid;
+      }
+      if (phase == kFind) continue;
+      goto resume;
     }
-    if (phase != kTrackVoxel && phase != kTrackBox && !(kFull && phase == kTrackMesh)) continue;
+    if (phase != kTrackVoxel && !(kFull && phase == kTrackMesh)) continue;
     {
 
     // ---- tracking inside solid ph.solid_id ----
     // the solid's and navigator's per-step fields in six 16-byte loads
     // (DevSolid / DevNavigator lead with them)
     const DevSolid& so = solids[ph.solid_id];
-    const int4 s3 = load4i(&so.number_of_voxels[0]);  // number_of_voxels xyz, navigator
+    const DevSolid& grid = kBatch && P.shared_grids ? scene_solids[ph.solid_id] : so;
+    const int4 s3 = load4i(&grid.number_of_voxels[0]);  // number_of_voxels xyz, navigator
     const int nav = s3.w;
     const int4 n0 = load4i(&navs[nav]);               // number_of_bins, process_pack, sigma / cut offsets
     const float4* sig = reinterpret_cast<const float4*>(tab.base + static_cast<uint32_t>(n0.z));
-    if (ph.E != cached_E || nav != cached_nav) {
-      energy_id = binary_search(ph.E, tab.energy_bins(nav), n0.x);
-      cached_E = ph.E;
-      cached_nav = nav;
-    }
+    find_energy(nav, n0.x);
 
     leaving = &so;
     const uint32_t pack = static_cast<uint32_t>(n0.y);
     if (!kFull || phase != kTrackMesh) {
-      // Up to kTrackSteps steps through a voxelized solid
-      // (track_through_ggems_voxelized_solid, TrackThroughGGEMSVoxelizedSolid.cl:133-310)
-      // or a detector box (track_through_ggems_solid_box,
-      // TrackThroughGGEMSSolidBox.cl:122-248): the same sampling and slab test
-      // against the current voxel or the whole box (a grid of one voxel of
-      // material 0), then each solid's own tail.  A step that neither leaves the
-      // solid nor interacts nor falls below a cut has no branch between the
-      // voxel index and its end, so that the label's load, the three draws and
-      // the slab test overlap; everything else is behind one test.
-      const bool voxel = phase == kTrackVoxel;
-      const float threshold = voxel ? 0.0f : so.threshold;
+      // Up to kTrackSteps steps through a voxelized solid that surely cross
+      // their voxel, which 97 % do: no logarithm, no branch between the voxel
+      // index and the step's end, so that the label's load, the three draws and
+      // the slab test overlap.  Any other step is left undone, its random state
+      // included, and taken as a whole in a round of the kInteract phase.  With a
+      // logarithm and a division per process in every step CBCT of 1e8 primaries
+      // took 270 ms, without 205 ms, and with the short forms below 172 ms.
+      //
+      // Every photon here is at least kTolerance inside the solid (the step's own
+      // test of its end, or the one before the loop), and the host has checked
+      // the grid for it (fast_steps in gg_runtime.cu).  That shortens three parts
+      // of the step without a bit's difference:
+      //  * a voxel index of such a position is in the grid;
+      //  * the position is inside its voxel up to a few roundings, all of them
+      //    below kTolerance, so safety_inside is a clamp;
+      //  * from at least kTolerance inside the voxel every axis has one face
+      //    behind and one ahead, so distance_to_aabb is the nearest face ahead.
+      //    Its test that the ray stays 2 kTolerance in the box can only fail for
+      //    a direction along x (else tmin is behind the photon, and two faces of
+      //    different axes are 2 sqrt(2) kTolerance apart along any ray): steps
+      //    shorter than that are left to the whole step.
       const float* cuts = reinterpret_cast<const float*>(tab.base + static_cast<uint32_t>(n0.w));
+      const int stride = row_stride(pack);
+      const uint8_t* labels = so.labels;
+      {
+        const float4 c = load4f(&grid.inv_voxel_sizes[2]), d = load4f(&grid.inner_max[0]);
+        if (!(ph.p.x >= c.y && ph.p.x <= d.x && ph.p.y >= c.z && ph.p.y <= d.y && ph.p.z >= c.w && ph.p.z <= d.z)) {
+          phase = kInteract;
+          continue;
+        }
+      }
 #pragma unroll 1
-      for (int k = 0; k < (kDose ? kTrackStepsDose : kTrackSteps); ++k) {
-        const float4 s0 = load4f(&so.border_min[0]);     // border_min xyz, border_max x
-        const float4 s1 = load4f(&so.border_max[1]);     // border_max yz, voxel_sizes xy
-        const float4 s2 = load4f(&so.voxel_sizes[2]);    // voxel_sizes z, inv_voxel_sizes xyz
-        const int4 s4 = load4i(&so.labels);              // labels (2 words)
-        const V3 bmin = v3(s0.x, s0.y, s0.z), bmax = v3(s0.w, s1.x, s1.y), vs = v3(s1.z, s1.w, s2.x);
-        const int nx = s3.x, ny = s3.y, nz = s3.z;
-        V3 q = sub(ph.p, bmin);
-        int ix, iy, iz;
-        V3 vmin, vmax;
-        bool outside;
-        if (P.voxel_mode != kVoxelGeneral) {
-          q = P.voxel_mode == kVoxelPow2 ? mul(q, v3(s2.y, s2.z, s2.w))
-                                         : v3(quotient(q.x, vs.x, s2.y), quotient(q.y, vs.y, s2.z), quotient(q.z, vs.z, s2.w));
-          // trunc(q) without the conversion pipe: 2^23 + q rounded towards
-          // zero holds trunc(q) in its low bits (and a q of 2^23 or more gives
-          // bits beyond any n); a q in (-1, 0) truncates to voxel 0, one of
-          // -1 or less is outside
-          const float mx = __fadd_rz(fmaxf(q.x, 0.0f), kTwo23), my = __fadd_rz(fmaxf(q.y, 0.0f), kTwo23),
-                      mz = __fadd_rz(fmaxf(q.z, 0.0f), kTwo23);
-          vmin = add(bmin, mul(v3(mx - kTwo23, my - kTwo23, mz - kTwo23), vs));
-          vmax = add(vmin, vs);
-          ix = __float_as_int(mx) - __float_as_int(kTwo23);
-          iy = __float_as_int(my) - __float_as_int(kTwo23);
-          iz = __float_as_int(mz) - __float_as_int(kTwo23);
-          outside = ix >= nx || iy >= ny || iz >= nz || fminf(fminf(q.x, q.y), q.z) <= -1.0f;
-        } else {
-          q = voxel ? divv(q, vs) : v3(0.0f, 0.0f, 0.0f);
-          ix = __float2int_rz(q.x);
-          iy = __float2int_rz(q.y);
-          iz = __float2int_rz(q.z);
-          outside = ix >= nx || iy >= ny || iz >= nz || ix < 0 || iy < 0 || iz < 0;
-          vmin = add(bmin, mul(v3(static_cast<float>(ix), static_cast<float>(iy), static_cast<float>(iz)), vs));
-          vmax = voxel ? add(vmin, vs) : bmax;
-        }
-        if (outside) {
-          ph.psd = kOutOfWorld;
-          ph.solid_id = -1;
-          leave = 1;
-          break;
-        }
-        const uint8_t* labels = reinterpret_cast<const uint8_t*>(
-            (static_cast<unsigned long long>(static_cast<uint32_t>(s4.y)) << 32) | static_cast<uint32_t>(s4.x));
-        const int material = __ldg(labels + (ix + iy * nx + iz * nx * ny));
-        int proc;
-        float nid = next_interaction(rng, pack, P.fast_sampling != 0,
-                                     sig + (material * n0.x + energy_id) * row_stride(pack), proc);
-        ph.p = safety_inside(ph.p, vmin, vmax);
-        const float dtb = distance_to_aabb(ph.p, ph.d, inv_d, vmin, vmax);
-        const bool crosses = dtb <= nid;
-        if (kDose && P.photon_tracking && crosses && voxel && so.dose_map >= 0) {
-          const DevDoseMap& dm = P.dose_maps[so.dose_map];
-          if (dm.photon_tracking) {
-            int id = dosel(dm, ph.p);
-            if (id >= 0) atomicAdd(dm.photon_tracking + id, 1);
-          }
-        }
-        nid = crosses ? dtb + kTolerance : nid;
-        proc = crosses ? GG_TRANSPORTATION : proc;
-        ph.p = safety_outside(add(ph.p, scale(ph.d, nid)), vmin, vmax);
-        const bool inside = in_aabb(ph.p, bmin, bmax);
-        const float cut = cuts[material];
-        if (kDose && P.tle && inside && voxel && so.dose_tle) {
-          // The step's deposit depends only on the energy before the interaction,
-          // so it is recorded here even when the interaction itself is deferred.
-          dose_record(P.dose_maps[so.dose_map], tle_edep(tab.attenuation(nav), material, ph.E, nid), ph.p);
-        }
-        if (kAux && inside) trk(GG_TRACK_STEP, ph.solid_id, proc);
-        if (inside && proc == GG_TRANSPORTATION && ph.E > cut && ph.E >= threshold) continue;
-        if (!inside) {
-          ph.psd = kOutOfWorld;
-          ph.solid_id = -1;
-          leave = 1;
-          break;
-        }
-        if (!voxel && ph.E < threshold) ph.status = GG_DEAD;
-        if (proc == GG_COMPTON_SCATTERING || proc == GG_RAYLEIGH_SCATTERING) {
-          pending = (proc << 8) | material;
+      for (int k = 0; k < kTrackSteps; ++k) {
+        const float4 a = load4f(&grid.border_min[0]);        // border_min xyz, voxel_sizes x
+        const float4 b = load4f(&grid.voxel_sizes[1]);       // voxel_sizes yz, inv_voxel_sizes xy
+        const float4 c = load4f(&grid.inv_voxel_sizes[2]);   // inv_voxel_sizes z, inner_min xyz
+        const float4 d = load4f(&grid.inner_max[0]);         // inner_max xyz, label_bias
+        const V3 bmin = v3(a.x, a.y, a.z), vs = v3(a.w, b.x, b.y);
+        const V3 r = sub(ph.p, bmin);
+        const V3 q = P.voxel_mode == kVoxelPow2 ? mul(r, v3(b.z, b.w, c.x))
+                                                : v3(quotient(r.x, vs.x, b.z), quotient(r.y, vs.y, b.w), quotient(r.z, vs.z, c.x));
+        // trunc(q) without the conversion pipe: 2^23 + q rounded towards zero
+        // holds trunc(q) in its low bits; label_bias takes the bits of the three
+        // 2^23 out of the label's index
+        const float mx = __fadd_rz(q.x, kTwo23), my = __fadd_rz(q.y, kTwo23), mz = __fadd_rz(q.z, kTwo23);
+        const uint32_t voxel = (__float_as_uint(mz) * static_cast<uint32_t>(s3.y) + __float_as_uint(my)) * static_cast<uint32_t>(s3.x) +
+                               __float_as_uint(mx) - __float_as_uint(d.w);
+        const int material = __ldg(labels + voxel);
+        const V3 vmin = add(bmin, mul(v3(mx - kTwo23, my - kTwo23, mz - kTwo23), vs));
+        const V3 vmax = add(vmin, vs);
+        Kiss next = rng;
+        const Draws draws = draw_processes(next, pack, P.fast_sampling != 0);
+        const V3 p = v3(fminf(fmaxf(ph.p.x, vmin.x + kTolerance), vmax.x - kTolerance),
+                        fminf(fmaxf(ph.p.y, vmin.y + kTolerance), vmax.y - kTolerance),
+                        fminf(fmaxf(ph.p.z, vmin.z + kTolerance), vmax.z - kTolerance));
+        const float dtb = fminf(fminf(fmaxf((vmin.x - p.x) * inv_d.x, (vmax.x - p.x) * inv_d.x),
+                                      fmaxf((vmin.y - p.y) * inv_d.y, (vmax.y - p.y) * inv_d.y)),
+                                fmaxf((vmin.z - p.z) * inv_d.z, (vmax.z - p.z) * inv_d.z));
+        const float4 sigma = sig[(material * n0.x + energy_id) * stride];
+        if (!(surely_crosses(draws, sigma, dtb) && dtb >= 2.0f * kTolerance && ph.E > cuts[material])) {
           phase = kInteract;
           break;
         }
-        if (!voxel) {
-          if (proc == GG_PHOTOELECTRIC_EFFECT) {
-            ph.status = GG_DEAD;
-            ph.E = 0.0f;
-            box_histogram(so, ph);
-          }
-        } else {
-          if (proc == GG_PHOTOELECTRIC_EFFECT) {
-            if (kDose && so.dose_map >= 0 && !so.dose_tle) dose_record(P.dose_maps[so.dose_map], ph.E, ph.p);
-            ph.status = GG_DEAD;
-            ph.E = 0.0f;
-          }
-          if (ph.E <= cut) {
-            if (kDose && so.dose_map >= 0) dose_record(P.dose_maps[so.dose_map], ph.E, ph.p);
-            ph.status = GG_DEAD;
-          }
-        }
-        if (ph.status == GG_DEAD) {
-          leave = 2;
+        rng = next;
+        ph.p = p;
+        if (!step_to(so, true, nav, material, dtb + kTolerance, GG_TRANSPORTATION, vmin, vmax, v3(c.y, c.z, c.w),
+                     v3(d.x, d.y, d.z))) {
+          ph.psd = kOutOfWorld;
+          ph.solid_id = -1;
+          leave = 1;
           break;
         }
       }
@@ -1446,7 +1545,8 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
         next = x.second;
       }
       int proc;
-      float nid = next_interaction(rng, pack, P.fast_sampling != 0, sig + energy_id * row_stride(pack), proc);
+      float nid = next_interaction(draw_processes(rng, pack, P.fast_sampling != 0), pack,
+                                   sig[energy_id * row_stride(pack)], proc);
       const float dx = next.x - ph.p.x, dy = next.y - ph.p.y, dz = next.z - ph.p.z;
       const float to_next = sqrtf(dx * dx + dy * dy + dz * dz);
       if (to_next <= nid) {
@@ -1463,7 +1563,7 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
       ph.p = add(ph.p, scale(ph.d, nid));
       trk(GG_TRACK_STEP, ph.solid_id, proc);
       if (proc == GG_COMPTON_SCATTERING || proc == GG_RAYLEIGH_SCATTERING) {
-        pending = proc << 8;
+        pending = proc;
         phase = kInteract;
         continue;
       }
@@ -1480,7 +1580,10 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
     } while (0);
     }
   exit_solid:
-    if (leave) leave_solid(*leaving, leave == 2);
+    if (leave) leave_solid(leaving, leave);
+    continue;
+  resume:
+    inv_d = reciprocal(ph.d);
   }
 }
 

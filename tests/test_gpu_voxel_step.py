@@ -1,0 +1,93 @@
+"""The transport kernel's short voxel step against its whole step.
+
+* surely_crosses() (CPU, float arithmetic): where it says that a photon crosses
+  its voxel, no process's -logf(u) / sigma is below the distance, with the
+  logarithm an ulp either way.
+* On the GPU a launch takes whole steps only when a grid of it is too long for
+  the short ones: the same histories, states and tallies bit for bit, for odd
+  voxel counts, voxel sizes with and without a power of two, a rotated phantom,
+  and a pencil beam along each axis of the grid.
+"""
+
+import math
+
+import numpy as np
+import pytest
+
+import parity
+import scenes
+
+F = np.float32
+
+
+def _fma(a, b, c):
+    return (a.astype(np.longdouble) * b.astype(np.longdouble) + c.astype(np.longdouble)).astype(F)
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_a_sure_crossing_has_no_nearer_interaction(seed):
+    rng = np.random.default_rng(seed)
+    n = 2_000_000
+    sigma = np.exp(rng.uniform(np.log(1e-12), np.log(1e3), n)).astype(F)
+    distance = np.exp(rng.uniform(np.log(5e-4), np.log(3e3), n)).astype(F)
+    draw = rng.integers(0, 1 << 32, n, dtype=np.uint64)
+    # half of the draws where the test's two sides meet
+    edge = (1.0 - sigma.astype(np.float64) * distance) * 2.0 ** 32 * (1.0 + rng.normal(0, 1e-6, n))
+    pick = (rng.random(n) < 0.5) & (edge > 0) & (edge < 2.0 ** 32)
+    draw[pick] = edge[pick].astype(np.uint64)
+    draw[:64] = np.arange(64)
+    draw[64:128] = (1 << 32) - 1 - np.arange(64)
+    x = draw.astype(np.uint32).astype(F)
+    reach = (distance * F(float.fromhex("0x1.00004p+32"))).astype(F)
+    sure = _fma(sigma, reach, x) < F(2.0 ** 32 - 2.0 ** 11)
+    assert 0.2 < sure.mean() < 0.9 and (sure & pick).any() and (~sure & pick).any()
+    u = _fma(x, np.full(n, float.fromhex("-0x1.ffp-56"), F), (x * F(2.0 ** -32)).astype(F))
+    with np.errstate(divide="ignore"):
+        log = (-np.log(u.astype(np.float64))).astype(F)
+    for a in (log, np.nextafter(log, F(0)), np.nextafter(log, F(np.inf))):
+        assert ((a / sigma)[sure] >= distance[sure]).all()
+
+
+def _scene(n, voxel, ops, dose, far_voxels):
+    sc = scenes.Scene()
+    t = sc.add_tables(scenes.Tables(["Air", "Water", "Bone185"]))
+    sc.add_voxelized(scenes.ellipsoid_phantom(n, voxel, seed=4), (voxel, voxel, voxel), t, ops=ops,
+                     dose={"photon_tracking": True} if dose else None)
+    # far off the beam; 1.28 mm long, or too long for the launch's short steps
+    far = np.ones((1, 1, far_voxels), np.uint8)
+    sc.add_voxelized(far, (0.02, 1.0, 1.0), t, ops=[("translation", (0.0, 5000.0, 0.0))])
+    sc.add_flat_detector(sc.add_tables(scenes.Tables(["GOS"])), (50, 40, 1), (8.0, 10.0, 10.0), 1500.0, 1000.0,
+                         F(10.0) * scenes.KEV)
+    return sc
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,voxel,rotation,dose,aperture", [
+    (33, 4.0, (0.0, 0.0, 0.0), False, 9.0),
+    (64, 2.0, (0.0, 0.0, 0.0), True, 9.0),
+    (41, 3.1, (0.0, 0.0, 0.3), True, 9.0),
+    (117, 0.7, (0.2, 0.1, 0.0), False, 4.0),
+    (40, 2.5, (0.0, 0.0, 0.0), True, 0.0),
+    (40, 2.5, (0.0, 0.0, math.pi / 2), True, 0.0),
+    (40, 2.5, (0.0, math.pi / 2, 0.0), False, 0.0),
+    (1, 60.0, (0.0, 0.0, 0.0), True, 2.0),
+])
+def test_short_steps_match_whole_ones(n, voxel, rotation, dose, aperture):
+    from ggems_b200 import _native
+    ctx = _native.Context(0)
+    try:
+        src = scenes.XRaySource(spectrum=scenes.synthetic_spectrum(), aperture_deg=aperture)
+        runs = [parity.run_gpu(ctx, _scene(n, voxel, [("rotation", rotation)], dose, far), src, 40000)
+                for far in (64, 1 << 17)]
+        (P0, T0, st0), (P1, T1, st1) = runs
+        assert T0.histograms[0].sum() > 0
+        assert parity.history_agreement(P0, P1)[0] == 1.0
+        assert np.array_equal(st0, st1)
+        for a, b in zip(T0.histograms, T1.histograms):
+            assert np.array_equal(a, b)
+        if dose:
+            assert T0.hit[0].sum() > 0
+            for name in ("edep", "hit", "photon_tracking"):
+                assert np.array_equal(getattr(T0, name)[0], getattr(T1, name)[0])
+    finally:
+        ctx.close()
