@@ -81,6 +81,11 @@ struct DevDoseMap {
   int32_t* photon_tracking;      // nullptr when not recorded
 };
 
+constexpr int kMeshNodeFloat4 = 8;    // 7 used: a node starts on a 128-byte line
+constexpr int kMeshLeaf = 8;          // most triangles of a leaf
+constexpr int kMeshStack = 96;        // entries of the walk's stack; the host checks the tree against it
+constexpr int kMeshNoChild = 0x7fffffff;
+
 struct alignas(16) DevSolid {
   // read by every tracking step: the first 88 bytes, vector loads
   float border_min[3];
@@ -107,10 +112,10 @@ struct alignas(16) DevSolid {
   // each ({min xyz, max x}, {max y, max z, first, count} with first / count as
   // int bits), and triangles grouped by node, 3 float4 each
   // ({p0 xyz, e1 x}, {e1 yz, e2 xy}, {e2 z, -, -, -}) with e1 = p1 - p0, e2 = p2 - p0.
-  // With mesh_bvh set, mesh_nodes is instead a bounding-volume hierarchy in
-  // the same 2-float4 form: count > 0 marks a leaf owning triangles
-  // [first, first + count), count == 0 an inner node whose children are
-  // first and first + 1.
+  // With mesh_bvh set, mesh_nodes is instead a bounding-volume hierarchy of
+  // kMeshNodeFloat4 float4 a node: min x of its four children, max x, min y,
+  // max y, min z, max z, and four int references: a node's index, ~(first
+  // triangle * kMeshLeaf + count - 1), or kMeshNoChild (with a box no ray hits).
   const float4* mesh_nodes;
   int32_t mesh_node_count;
   const float4* mesh_triangles;

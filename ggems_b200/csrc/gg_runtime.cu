@@ -12,6 +12,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <limits>
 #include <map>
 #include <mutex>
 #include <random>
@@ -215,7 +216,7 @@ float int_bits(int x) {
 
 // Bounding-volume hierarchy over the mesh triangles: binned surface-area
 // heuristic (12 bins on the widest centroid axis), leaves of at most 4
-// triangles, depth at most 48 (the device walk keeps a 64-entry stack).
+// triangles, depth at most 48.  Two children a node, for wide_bvh.
 // Boxes are grown by a relative 1e-5 plus 1e-4 mm so that rounding in the
 // slab test never prunes a triangle the ray actually crosses.
 void build_bvh(const gg_solid& g, std::vector<float4>* nodes_out, std::vector<float4>* tris_out) {
@@ -333,6 +334,88 @@ void build_bvh(const gg_solid& g, std::vector<float4>* nodes_out, std::vector<fl
       tris_out->push_back(triangle_record(g.triangles + static_cast<size_t>(order[i]) * GG_TRIANGLE_FLOATS, part));
 }
 
+// The device form of build_bvh's hierarchy (gg_internal.cuh): inner nodes pulled
+// up into their parents until each has `width` children (the largest first, in
+// the hierarchy's order).  A child's padded box lies in its parent's, so the
+// leaves whose boxes a ray hits are the same whatever nodes lie above them.
+// Returns the most stack entries that a walk of it needs.
+int wide_bvh(const std::vector<float4>& binary, int width, std::vector<float4>* out) {
+  struct Child {
+    int node;            // of the binary hierarchy; its box
+    int first, count;    // triangles (count 0: an inner node)
+  };
+  auto bits = [](float f) {
+    int i;
+    std::memcpy(&i, &f, 4);
+    return i;
+  };
+  auto child_of = [&](int node) { return Child{node, bits(binary[2 * node + 1].z), bits(binary[2 * node + 1].w)}; };
+  auto area = [&](int node) {
+    const float4 a = binary[2 * node], b = binary[2 * node + 1];
+    const float x = a.w - a.x, y = b.x - a.y, z = b.y - a.z;
+    return x * y + y * z + z * x;
+  };
+  auto open = [&](const Child& c, std::vector<Child>* to) {
+    if (c.count == 0) {
+      to->push_back(child_of(c.first));
+      to->push_back(child_of(c.first + 1));
+    } else {  // more triangles than a leaf holds (the hierarchy's depth limit): halves in the same box
+      const int half = c.count / 2;
+      to->push_back(Child{c.node, c.first, half});
+      to->push_back(Child{c.node, c.first + half, c.count - half});
+    }
+  };
+  auto is_leaf = [](const Child& c) { return c.count > 0 && c.count <= gg::kMeshLeaf; };
+  struct Item {
+    Child from;
+    int node, stack;
+  };
+  constexpr int kFields = gg::kMeshNodeFloat4;
+  out->assign(kFields, make_float4(0, 0, 0, 0));
+  std::vector<Item> work{{child_of(0), 0, 0}};
+  int deepest = 0;
+  while (!work.empty()) {
+    const Item it = work.back();
+    work.pop_back();
+    std::vector<Child> c;
+    if (is_leaf(it.from)) c.push_back(it.from);  // a mesh of one leaf
+    else open(it.from, &c);
+    for (;;) {
+      int widest = -1;
+      for (int i = 0; i < static_cast<int>(c.size()); ++i)
+        if (!is_leaf(c[i]) && (widest < 0 || area(c[i].node) > area(c[widest].node))) widest = i;
+      if (widest < 0 || static_cast<int>(c.size()) >= width) break;
+      std::vector<Child> halves;
+      open(c[widest], &halves);
+      c[widest] = halves[0];
+      c.insert(c.begin() + widest + 1, halves[1]);
+    }
+    const int stack = it.stack + static_cast<int>(c.size()) - 1;
+    deepest = std::max(deepest, stack);
+    float field[6][4];
+    int ref[4];
+    for (int i = 0; i < 4; ++i) {
+      for (auto& f : field) f[i] = std::numeric_limits<float>::infinity();
+      ref[i] = gg::kMeshNoChild;
+      if (i >= static_cast<int>(c.size())) continue;
+      const float4 a = binary[2 * c[i].node], b = binary[2 * c[i].node + 1];
+      const float box[6] = {a.x, a.w, a.y, b.x, a.z, b.y};
+      for (int f = 0; f < 6; ++f) field[f][i] = box[f];
+      if (is_leaf(c[i])) {
+        ref[i] = ~(c[i].first * gg::kMeshLeaf + c[i].count - 1);
+      } else {
+        ref[i] = static_cast<int>(out->size() / kFields);
+        out->resize(out->size() + kFields, make_float4(0, 0, 0, 0));
+        work.push_back({c[i], ref[i], stack});
+      }
+    }
+    float4* n = out->data() + static_cast<size_t>(kFields) * it.node;
+    for (int f = 0; f < 6; ++f) n[f] = make_float4(field[f][0], field[f][1], field[f][2], field[f][3]);
+    std::memcpy(n + 6, ref, sizeof(ref));
+  }
+  return deepest;
+}
+
 // Whether meshed solids use the hierarchy: GGEMS_B200_MESH_BVH = 0 (never:
 // GGEMS's octree scan), 1 (always), unset (meshes above 4096 triangles).
 bool use_bvh(int triangles) {
@@ -352,7 +435,13 @@ int upload_mesh(gg_context* c, const gg_solid& g, gg::DevSolid* d, std::vector<v
   std::vector<float4> nodes, tris;
   d->mesh_bvh = use_bvh(g.number_of_triangles) ? 1 : 0;
   if (d->mesh_bvh) {
-    build_bvh(g, &nodes, &tris);
+    std::vector<float4> binary;
+    build_bvh(g, &binary, &tris);
+    // Four children where the stack holds a walk of that; two (at most one entry
+    // a level, and few levels more for oversized leaves) for degenerate meshes.
+    if (g.number_of_triangles >= (1 << 28)) return fail(GG_ERROR_INVALID_ARGUMENT, "mesh of more than 2^28 triangles");
+    if (wide_bvh(binary, 4, &nodes) > gg::kMeshStack && wide_bvh(binary, 2, &nodes) > gg::kMeshStack)
+      return fail(GG_ERROR_INVALID_ARGUMENT, "mesh hierarchy deeper than the walk's stack");
     float4* dn;
     float4* dt;
     int rc;
@@ -360,7 +449,7 @@ int upload_mesh(gg_context* c, const gg_solid& g, gg::DevSolid* d, std::vector<v
         (rc = dev_copy_to(c, owner, tris.data(), tris.size(), &dt)))
       return rc;
     d->mesh_nodes = dn;
-    d->mesh_node_count = static_cast<int32_t>(nodes.size() / 2);
+    d->mesh_node_count = static_cast<int32_t>(nodes.size() / gg::kMeshNodeFloat4);
     d->mesh_triangles = dt;
     return GG_OK;
   }

@@ -655,9 +655,10 @@ __device__ __forceinline__ bool ray_hits_box(const float pos[3], const float dir
 // rule; the search ends at 16 crossings (GGEMS writes past its array beyond
 // that).  Octree form: every node that owns triangles, in node order, is
 // slab-tested and its triangles intersected, exactly GGEMS's scan.  BVH form
-// (large meshes): the hierarchy is walked with a stack; each triangle test is
-// the same arithmetic, so the crossings found are the same set and only their
-// discovery order (hence exact ties) can differ from the scan's.
+// (large meshes): a hierarchy of four children a node is walked in order with a
+// stack; each triangle test is the same arithmetic, so the crossings found are
+// the same set and only their discovery order (hence exact ties) can differ from
+// the scan's.
 __device__ __noinline__ MeshCrossings mesh_crossings(V3 p, V3 d, V3 inv, const float4* nodes, int node_count,
                                                      const float4* tris, int bvh) {
   MeshCrossings out;
@@ -676,25 +677,59 @@ __device__ __noinline__ MeshCrossings mesh_crossings(V3 p, V3 d, V3 inv, const f
     }
     return out;
   }
-  constexpr int kStack = 64;
-  int stack[kStack];
-  int sp = 0, node = 0;
+  // A lane walks down to its next leaf, then all lanes that have one test their
+  // triangles together.  What bounds the walk is divergence (lanes leave it after
+  // different numbers of nodes and leaves: 5 of 32 active) and the chain of node
+  // loads.  Four boxes a node halve both against two children with a box tested
+  // per step: 245,760 triangles, 1e7 primaries 80.5 -> 52.8 ms (under the
+  // profiler 2e6 primaries 16.3 -> 10.5 ms, 22 % fewer warp instructions, issue
+  // slots 52 -> 63 % busy).
+  int stack[kMeshStack];
+  int sp = 0, ref = 0;
+  const bool along = fabsf(d.x) < kEps6 || fabsf(d.y) < kEps6 || fabsf(d.z) < kEps6;
   for (;;) {
-    const float4 a = __ldg(nodes + 2 * node), b = __ldg(nodes + 2 * node + 1);
-    const float mn[3] = {a.x, a.y, a.z}, mx[3] = {a.w, b.x, b.y};
-    if (ray_hits_box(pos, dir, ood, mn, mx)) {
-      const int first = __float_as_int(b.z), count = __float_as_int(b.w);
-      if (count > 0) {
-        for (int k = first; k < first + count; ++k)
-          if (add_crossing(p, d, tris, k, out, c)) return out;
-      } else if (sp < kStack) {
-        stack[sp++] = first + 1;
-        node = first;
-        continue;
+    while (ref >= 0 && ref != kMeshNoChild) {
+      const float4* n = nodes + static_cast<size_t>(kMeshNodeFloat4) * ref;
+      const float4 lx = __ldg(n), hx = __ldg(n + 1), ly = __ldg(n + 2), hy = __ldg(n + 3), lz = __ldg(n + 4), hz = __ldg(n + 5);
+      const int4 child = __ldg(reinterpret_cast<const int4*>(n + 6));
+      auto hit = [&](float x0, float x1, float y0, float y1, float z0, float z1) -> bool {
+        if (along) {
+          const float mn[3] = {x0, y0, z0}, mx[3] = {x1, y1, z1};
+          return ray_hits_box(pos, dir, ood, mn, mx);
+        }
+        // ray_hits_box without its tests for a direction along a face; its early
+        // returns only save work (tmin grows, tmax shrinks)
+        const float ax = (x0 - p.x) * inv.x, bx = (x1 - p.x) * inv.x, ay = (y0 - p.y) * inv.y, by = (y1 - p.y) * inv.y,
+                    az = (z0 - p.z) * inv.z, bz = (z1 - p.z) * inv.z;
+        const float tmin = fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fmaxf(fminf(az, bz), 0.0f));
+        const float tmax = fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fminf(fmaxf(az, bz), FLT_MAX));
+        return !(tmin > tmax);
+      };
+      // the first child hit is next, the others wait on the stack, the last one at the bottom
+      int next = kMeshNoChild;
+      if (hit(lx.w, hx.w, ly.w, hy.w, lz.w, hz.w)) next = child.w;
+      if (hit(lx.z, hx.z, ly.z, hy.z, lz.z, hz.z)) {
+        if (next != kMeshNoChild) stack[sp++] = next;
+        next = child.z;
       }
+      if (hit(lx.y, hx.y, ly.y, hy.y, lz.y, hz.y)) {
+        if (next != kMeshNoChild) stack[sp++] = next;
+        next = child.y;
+      }
+      if (hit(lx.x, hx.x, ly.x, hy.x, lz.x, hz.x)) {
+        if (next != kMeshNoChild) stack[sp++] = next;
+        next = child.x;
+      }
+      if (next == kMeshNoChild && sp > 0) next = stack[--sp];
+      ref = next;
     }
-    if (sp == 0) break;
-    node = stack[--sp];
+    if (ref == kMeshNoChild) break;
+    const int first = static_cast<int>(static_cast<uint32_t>(~ref) / kMeshLeaf);
+    const int end = first + static_cast<int>(static_cast<uint32_t>(~ref) % kMeshLeaf) + 1;
+#pragma unroll 1
+    for (int k = first; k < end; ++k)
+      if (add_crossing(p, d, tris, k, out, c)) return out;
+    ref = sp > 0 ? stack[--sp] : kMeshNoChild;
   }
   return out;
 }
