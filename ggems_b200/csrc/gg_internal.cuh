@@ -33,7 +33,7 @@ constexpr double kEdepScale = 4294967296.0;
 // multiply-adds instead of a division) is proven: no overflow, no subnormal
 // remainder for the operands transport divides.
 constexpr float kQuotientMin = 1.0e-25f, kQuotientMax = 1.0e25f;
-constexpr uint32_t kPackCount = 0x7fu, kPackReciprocals = 0x80u;
+constexpr uint32_t kPackCount = 0xffu;
 // Voxel index of a solid: general (divisions, integer conversions),
 // multiplication by an exact 2^-k, or quotient() with the correctly rounded
 // reciprocal; the last two for at most 2^22 voxels an axis (trunc by rounding
@@ -42,17 +42,13 @@ constexpr uint32_t kPackCount = 0x7fu, kPackReciprocals = 0x80u;
 // of its voxelized solids needs; general: whole steps only.  A box takes whole
 // steps too, as a grid of one voxel.
 constexpr int kVoxelGeneral = 0, kVoxelPow2 = 1, kVoxelReciprocal = 2, kVoxelBox = 3;
-// Tables with reciprocals may take this much of a block's shared memory: three
-// blocks of 256 threads with the photon stash stay resident per SM.  Larger
-// ones keep plain rows and divide.
-constexpr uint32_t kReciprocalTableBytes = 44 * 1024;
 
 struct alignas(16) DevNavigator {
   // read by every tracking step: the first 16 bytes, one vector load
   int32_t number_of_bins;
-  uint32_t process_pack;         // number_of_processes (kPackCount) | kPackReciprocals | process_id[i] << 8 (i + 1)
+  uint32_t process_pack;         // number_of_processes (kPackCount) | process_id[i] << 8 (i + 1)
   // byte offsets into the table blob (shared memory copy when it fits)
-  uint32_t sigma_offset;         // float4[number_of_materials * number_of_bins] (or [...][2] with the reciprocals)
+  uint32_t sigma_offset;         // float4[number_of_materials * number_of_bins]
   uint32_t photon_cut_offset;    // float[number_of_materials]
   int32_t number_of_materials;
   int32_t number_of_processes;
@@ -194,8 +190,8 @@ struct TransportParams {
   int32_t tracking_capacity;
   gg_track_point* tracking_points;
   int32_t* tracking_count;
-  int32_t voxel_mode;               // kVoxelGeneral, kVoxelReciprocal or kVoxelPow2: what serves every solid of the launch
-  int32_t fast_sampling;            // every navigator: all three processes, sigma rows with reciprocals
+  int32_t voxel_mode;               // kVoxelGeneral, kVoxelReciprocal or kVoxelPow2: what serves every voxelized solid of the launch
+  int32_t three_processes;          // every navigator has all three
   int32_t shared_grids;             // batched launch: every job's voxelized solids have the first job's grids
   int32_t photon_tracking;          // some dose map counts photons
   int32_t tle;                      // some dose map uses the track-length estimator

@@ -760,25 +760,6 @@ GG_API int gg_upload_scene(gg_context* c, const gg_scene* sc) {
       nav_tle[g.navigator] = 1;
   }
 
-  // Rows with reciprocals: every cross section 0 or within quotient()'s range,
-  // and the whole set small enough (kReciprocalTableBytes).
-  bool with_reciprocals = true;
-  size_t reciprocal_bytes = 0;
-  for (int n = 0; n < sc->number_of_tables && with_reciprocals; ++n) {
-    const gg_physics_tables& t = sc->tables[n];
-    const size_t cells = static_cast<size_t>(std::max(t.number_of_materials, 0)) * std::max(t.number_of_bins, 0);
-    reciprocal_bytes += cells * 32 + static_cast<size_t>(std::max(t.number_of_bins, 0)) * 4;
-    if (nav_tle[n]) reciprocal_bytes += (1 + static_cast<size_t>(std::max(t.number_of_materials, 0))) * GG_ATTENUATION_BINS * 4;
-    with_reciprocals = reciprocal_bytes <= gg::kReciprocalTableBytes;
-    for (int p = 0; p < std::min(t.number_of_processes, 3) && with_reciprocals; ++p) {
-      if (t.process_id[p] < 0 || t.process_id[p] > 2) break;  // refused below
-      for (size_t i = 0; i < cells && with_reciprocals; ++i) {
-        const float s = t.cross_sections[t.process_id[p] * cells + i];
-        with_reciprocals = s == 0.0f || (s >= gg::kQuotientMin && s <= gg::kQuotientMax);
-      }
-    }
-  }
-
   // ---- tables: shared-memory blob + HBM element data ----
   std::vector<unsigned char> blob;
   std::vector<gg::DevNavigator> navs(sc->number_of_tables);
@@ -802,18 +783,13 @@ GG_API int gg_upload_scene(gg_context* c, const gg_scene* sc) {
     blob.resize(align16(d.energy_bins_offset + nb * 4), 0);
     std::memcpy(blob.data() + d.energy_bins_offset, t.energy_bins, nb * 4);
     d.sigma_offset = static_cast<uint32_t>(blob.size());
-    blob.resize(d.sigma_offset + nm * nb * (with_reciprocals ? 32 : 16), 0);
+    blob.resize(d.sigma_offset + nm * nb * 16, 0);
     float* sig = reinterpret_cast<float*>(blob.data() + d.sigma_offset);
     const size_t block = static_cast<size_t>(nm) * nb;
-    const uint32_t row = with_reciprocals ? 8 : 4;
     for (uint32_t m = 0; m < nm; ++m)
       for (uint32_t b = 0; b < nb; ++b)
-        for (int p = 0; p < t.number_of_processes; ++p) {
-          const float s = t.cross_sections[t.process_id[p] * block + b + nb * m];
-          sig[(m * nb + b) * row + p] = s;
-          if (with_reciprocals) sig[(m * nb + b) * row + 4 + p] = 1.0f / s;
-        }
-    if (with_reciprocals) d.process_pack |= gg::kPackReciprocals;
+        for (int p = 0; p < t.number_of_processes; ++p)
+          sig[(m * nb + b) * 4 + p] = t.cross_sections[t.process_id[p] * block + b + nb * m];
     d.photon_cut_offset = static_cast<uint32_t>(blob.size());
     blob.resize(align16(d.photon_cut_offset + nm * 4), 0);
     std::memcpy(blob.data() + d.photon_cut_offset, t.photon_energy_cut, nm * 4);
@@ -1133,8 +1109,8 @@ int prepare_jobs(gg_context* c, const gg_job* jobs, int32_t n, std::vector<void*
     if (job_solids[i].type == GG_SOLID_VOXELIZED || first.type == GG_SOLID_VOXELIZED)
       P.shared_grids &= std::memcmp(&job_solids[i], &first, offsetof(gg::DevSolid, labels)) == 0 ? 1 : 0;
   }
-  P.fast_sampling = 1;
-  for (uint32_t pack : c->process_pack) P.fast_sampling &= (pack & 0xffu) == (3u | gg::kPackReciprocals) ? 1 : 0;
+  P.three_processes = 1;
+  for (uint32_t pack : c->process_pack) P.three_processes &= (pack & gg::kPackCount) == 3u ? 1 : 0;
   for (const gg::DevDoseMap& m : c->dose_host) P.photon_tracking |= m.photon_tracking ? 1 : 0;
   for (char t : c->dose_tle) P.tle |= t ? 1 : 0;
   P.regroup_lanes = c->regroup_lanes;

@@ -266,12 +266,13 @@ __device__ __forceinline__ float quotient(float a, float b, float y) {
 
 // The draws of one GetPhotonNextInteraction call before their conversion to
 // (0, 1): one per process, in process order (0 where a process is missing).
+// three: every navigator of the launch has all three processes.
 struct Draws {
   float x0, x1, x2;
 };
-__device__ __forceinline__ Draws draw_processes(Kiss& rng, uint32_t process_pack, bool fast) {
+__device__ __forceinline__ Draws draw_processes(Kiss& rng, uint32_t process_pack, bool three) {
   Draws w{0.0f, 0.0f, 0.0f};
-  if (fast) {
+  if (three) {
     w.x0 = rng.raw();
     w.x1 = rng.raw();
     w.x2 = rng.raw();
@@ -321,8 +322,6 @@ __device__ __forceinline__ float next_interaction(Draws w, uint32_t process_pack
   }
   return nid;
 }
-// Float4s a row of the sigma table takes.
-__device__ __forceinline__ int row_stride(uint32_t process_pack) { return (process_pack & kPackReciprocals) ? 2 : 1; }
 
 // 16-byte shared-memory (or global) loads of a struct's leading fields.
 __device__ __forceinline__ float4 load4f(const void* p) { return *reinterpret_cast<const float4*>(p); }
@@ -404,10 +403,9 @@ __device__ __noinline__ Interaction rayleigh(Interaction in, const DevNavigator&
   int mixture = nv.element_offset[material];
   int z = nv.atomic_number[mixture + n_minus_one];
   if (n_minus_one > 0) {
-    const int stride = row_stride(nv.process_pack);
-    const float4* row = sig + static_cast<size_t>(material * nb + energy_id) * stride;
+    const float4* row = sig + static_cast<size_t>(material * nb + energy_id);
     const int slot = nv.process_id[0] == GG_RAYLEIGH_SCATTERING ? 0 : (nv.process_id[1] == GG_RAYLEIGH_SCATTERING ? 1 : 2);
-    float kcs = lerp_ref(ebins[energy_id], pick(row[0], slot), ebins[energy_id + 1], pick(row[stride], slot), E0);
+    float kcs = lerp_ref(ebins[energy_id], pick(row[0], slot), ebins[energy_id + 1], pick(row[1], slot), E0);
     float x = rng.uniform() * kcs;
     float cs = 0.0f;
 #pragma unroll 1
@@ -557,9 +555,10 @@ __device__ __noinline__ PrimaryOut new_primary(Kiss rng, const DevSource& s) {
 // Track-length-estimator deposit of one voxel step
 // (TrackThroughGGEMSVoxelizedSolid.cl:286-301): E * mu_en(E, material) * step
 // (mm -> cm), with mu_en interpolated in the 220-bin attenuation table.
-__device__ __forceinline__ float tle_edep(const float* att, int material, float energy, float step) {
+// e_index: the energy's bin there, which a photon keeps between interactions:
+// searched once per run of steps, not per step.
+__device__ __forceinline__ float tle_edep(const float* att, int material, int e_index, float energy, float step) {
   const float* me = att + GG_ATTENUATION_BINS * (1 + material);
-  int e_index = binary_search(energy, att, GG_ATTENUATION_BINS);
   float mu_en = e_index == 0 ? me[0] : lerp_ref(att[e_index - 1], me[e_index - 1], att[e_index], me[e_index], energy);
   return energy * mu_en * step * 0.1f;
 }
@@ -902,7 +901,7 @@ constexpr int transport_registers(int blocks) { return (65536 / (kBlockThreads *
 
 template <bool kFull, bool kBatch, bool kDose, bool kAux, int kStash>
 __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch && kDose) || kStash == 2 ? 3 : 4))))
-    transport_kernel(TransportParams P) {
+    transport_kernel(const __grid_constant__ TransportParams P) {
   // shared memory: [tables][solids][navigators][mbarrier][stash]
   unsigned char* tables = g_smem;
   DevSolid* scene_solids = reinterpret_cast<DevSolid*>(g_smem + (P.tables_in_smem ? P.table_bytes : 0));
@@ -1043,11 +1042,15 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
     cached_E = ph.E;
     cached_nav = nav;
   };
+  auto find_tle_bin = [&](const DevSolid& so, int nav) -> int {
+    return kDose && P.tle && so.dose_tle ? binary_search(ph.E, tab.attenuation(nav), GG_ATTENUATION_BINS) : 0;
+  };
   // Moves the photon to the end of a step of length nid in a voxelized solid's
   // voxel or a detector box; whether that is inside the solid.
   // inner_min, inner_max: the solid's borders kTolerance inside (in_aabb's bounds).
-  auto step_to = [&](const DevSolid& so, bool voxel, int nav, int material, float nid, int proc, V3 vmin, V3 vmax,
-                     V3 inner_min, V3 inner_max) -> bool {
+  // tle_bin: tle_edep's e_index, where the solid's dose map uses it.
+  auto step_to = [&](const DevSolid& so, bool voxel, int nav, int material, int tle_bin, float nid, int proc, V3 vmin,
+                     V3 vmax, V3 inner_min, V3 inner_max) -> bool {
     if (kDose && P.photon_tracking && proc == GG_TRANSPORTATION && voxel && so.dose_map >= 0) {
       const DevDoseMap& dm = P.dose_maps[so.dose_map];
       if (dm.photon_tracking) {
@@ -1061,7 +1064,7 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
     if (kDose && P.tle && inside && voxel && so.dose_tle) {
       // The step's deposit depends only on the energy before the interaction,
       // so it is recorded here even when an interaction follows.
-      dose_record(P.dose_maps[so.dose_map], tle_edep(tab.attenuation(nav), material, ph.E, nid), ph.p);
+      dose_record(P.dose_maps[so.dose_map], tle_edep(tab.attenuation(nav), material, tle_bin, ph.E, nid), ph.p);
     }
     if (kAux && inside) trk(GG_TRACK_STEP, ph.solid_id, proc);
     return inside;
@@ -1319,16 +1322,16 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
           material = __ldg(so.labels + (ix + iy * nx + iz * nx * ny));
           const float4* row =
               reinterpret_cast<const float4*>(tab.base + static_cast<uint32_t>(n0.z)) +
-              (material * n0.x + energy_id) * row_stride(pack);
+              (material * n0.x + energy_id);
           const float cut = reinterpret_cast<const float*>(tab.base + static_cast<uint32_t>(n0.w))[material];
-          float nid = next_interaction(draw_processes(rng, pack, P.fast_sampling != 0), pack, row[0], proc);
+          float nid = next_interaction(draw_processes(rng, pack, P.three_processes != 0), pack, row[0], proc);
           ph.p = safety_inside(ph.p, vmin, vmax);
           const float dtb = distance_to_aabb(ph.p, ph.d, inv_d, vmin, vmax);
           if (dtb <= nid) {
             nid = dtb + kTolerance;
             proc = GG_TRANSPORTATION;
           }
-          if (!step_to(so, voxel, nav, material, nid, proc, vmin, vmax,
+          if (!step_to(so, voxel, nav, material, find_tle_bin(so, nav), nid, proc, vmin, vmax,
                        v3(so.inner_min[0], so.inner_min[1], so.inner_min[2]),
                        v3(so.inner_max[0], so.inner_max[1], so.inner_max[2]))) {
             ph.psd = kOutOfWorld;
@@ -1510,8 +1513,8 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
       //    different axes are 2 sqrt(2) kTolerance apart along any ray): steps
       //    shorter than that are left to the whole step.
       const float* cuts = reinterpret_cast<const float*>(tab.base + static_cast<uint32_t>(n0.w));
-      const int stride = row_stride(pack);
       const uint8_t* labels = so.labels;
+      const int tle_bin = find_tle_bin(so, nav);
       {
         const float4 c = load4f(&grid.inv_voxel_sizes[2]), d = load4f(&grid.inner_max[0]);
         if (!(ph.p.x >= c.y && ph.p.x <= d.x && ph.p.y >= c.z && ph.p.y <= d.y && ph.p.z >= c.w && ph.p.z <= d.z)) {
@@ -1539,21 +1542,21 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
         const V3 vmin = add(bmin, mul(v3(mx - kTwo23, my - kTwo23, mz - kTwo23), vs));
         const V3 vmax = add(vmin, vs);
         Kiss next = rng;
-        const Draws draws = draw_processes(next, pack, P.fast_sampling != 0);
+        const Draws draws = draw_processes(next, pack, P.three_processes != 0);
         const V3 p = v3(fminf(fmaxf(ph.p.x, vmin.x + kTolerance), vmax.x - kTolerance),
                         fminf(fmaxf(ph.p.y, vmin.y + kTolerance), vmax.y - kTolerance),
                         fminf(fmaxf(ph.p.z, vmin.z + kTolerance), vmax.z - kTolerance));
         const float dtb = fminf(fminf(fmaxf((vmin.x - p.x) * inv_d.x, (vmax.x - p.x) * inv_d.x),
                                       fmaxf((vmin.y - p.y) * inv_d.y, (vmax.y - p.y) * inv_d.y)),
                                 fmaxf((vmin.z - p.z) * inv_d.z, (vmax.z - p.z) * inv_d.z));
-        const float4 sigma = sig[(material * n0.x + energy_id) * stride];
+        const float4 sigma = sig[material * n0.x + energy_id];
         if (!(surely_crosses(draws, sigma, dtb) && dtb >= 2.0f * kTolerance && ph.E > cuts[material])) {
           phase = kInteract;
           break;
         }
         rng = next;
         ph.p = p;
-        if (!step_to(so, true, nav, material, dtb + kTolerance, GG_TRANSPORTATION, vmin, vmax, v3(c.y, c.z, c.w),
+        if (!step_to(so, true, nav, material, tle_bin, dtb + kTolerance, GG_TRANSPORTATION, vmin, vmax, v3(c.y, c.z, c.w),
                      v3(d.x, d.y, d.z))) {
           ph.psd = kOutOfWorld;
           ph.solid_id = -1;
@@ -1580,8 +1583,8 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
         next = x.second;
       }
       int proc;
-      float nid = next_interaction(draw_processes(rng, pack, P.fast_sampling != 0), pack,
-                                   sig[energy_id * row_stride(pack)], proc);
+      float nid = next_interaction(draw_processes(rng, pack, P.three_processes != 0), pack,
+                                   sig[energy_id], proc);
       const float dx = next.x - ph.p.x, dy = next.y - ph.p.y, dz = next.z - ph.p.z;
       const float to_next = sqrtf(dx * dx + dy * dy + dz * dz);
       if (to_next <= nid) {
