@@ -152,24 +152,34 @@ cudaError_t staged(int device, cudaStream_t stream, Block* block, const std::vec
   return error.load() != cudaSuccess ? static_cast<cudaError_t>(error.load()) : e;
 }
 
-// Whether the driver copies straight from or to this host address; *mapped: the
-// device's address of it, if it has one.
-bool page_locked(const void* host, void** mapped = nullptr) {
-  cudaPointerAttributes a{};
-  const bool known = cudaPointerGetAttributes(&a, host) == cudaSuccess && a.type != cudaMemoryTypeUnregistered;
-  cudaGetLastError();  // an address unknown to CUDA is not an error here
-  if (mapped) *mapped = known && a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
-  return known;
+// Whether the driver copies straight from or to this host array.  An array of
+// which only one end is page-locked is refused, as the driver refuses it.
+cudaError_t is_page_locked(const void* host, size_t bytes, bool* locked) {
+  const auto known = [](const void* p) {
+    cudaPointerAttributes a{};
+    const bool k = cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type != cudaMemoryTypeUnregistered;
+    cudaGetLastError();  // an address unknown to CUDA is not an error here
+    return k;
+  };
+  *locked = known(host);
+  return *locked == known(static_cast<const unsigned char*>(host) + bytes - 1) ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-void host_fixed_to_double(void* host, size_t bytes) {
-  unsigned char* p = static_cast<unsigned char*>(host);
-  for (size_t i = 0; i + 8 <= bytes; i += 8) {
-    long long v;
-    std::memcpy(&v, p + i, 8);
-    const double d = static_cast<double>(v) / kEdepScale;
-    std::memcpy(p + i, &d, 8);
+// One array by the copy engine, energies in pieces that the scratch holds.
+// Nothing but the driver's copies writes to the caller's array: they check its
+// whole range where it is page-locked.
+cudaError_t queue_copy(const HostCopy& c, void* scratch, size_t scratch_bytes, cudaStream_t stream) {
+  if (!c.fixed_point) return cudaMemcpyAsync(c.host, c.device, c.bytes, cudaMemcpyDeviceToHost, stream);
+  scratch_bytes &= ~static_cast<size_t>(7);
+  if (!scratch || scratch_bytes == 0) return cudaErrorInvalidValue;
+  for (size_t at = 0; at < c.bytes; at += scratch_bytes) {
+    const size_t bytes = std::min(scratch_bytes, c.bytes - at);
+    cudaError_t e = fixed_to_double(static_cast<const unsigned char*>(c.device) + at, scratch, bytes, stream);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(static_cast<unsigned char*>(c.host) + at, scratch, bytes, cudaMemcpyDeviceToHost, stream);
+    if (e != cudaSuccess) return e;
   }
+  return cudaSuccess;
 }
 
 }  // namespace
@@ -184,12 +194,11 @@ cudaError_t copies_to_host(int device, cudaStream_t stream, const HostCopy* copi
     std::vector<HostCopy> through;
     for (int i = 0; i < count; ++i) {
       if (copies[i].bytes == 0) continue;
-      if (page_locked(copies[i].host)) {
-        plain.push_back(copies[i]);
-      } else {
-        through.push_back(copies[i]);
-        total += copies[i].bytes;
-      }
+      bool locked = false;
+      const cudaError_t known = is_page_locked(copies[i].host, copies[i].bytes, &locked);
+      if (known != cudaSuccess) return known;
+      (locked ? plain : through).push_back(copies[i]);
+      if (!locked) total += copies[i].bytes;
     }
     if (total >= kStagedCopyBytes) block = lease(device);
     for (const HostCopy& c : through) {
@@ -204,36 +213,25 @@ cudaError_t copies_to_host(int device, cudaStream_t stream, const HostCopy* copi
     return cudaErrorMemoryAllocation;
   }
   cudaError_t e = cudaSuccess;
-  for (HostCopy& c : plain) {
-    void* mapped = nullptr;
-    const void* from = c.device;
-    if (c.fixed_point && page_locked(c.host, &mapped) && mapped && reinterpret_cast<uintptr_t>(mapped) % 8 == 0) {
-      if (e == cudaSuccess) e = fixed_to_double(c.device, mapped, c.bytes, stream);
-      c.fixed_point = false;
-      continue;
-    }
-    if (c.fixed_point && scratch && c.bytes <= scratch_bytes) {
-      if (e == cudaSuccess) e = fixed_to_double(c.device, scratch, c.bytes, stream);
-      from = scratch;
-      c.fixed_point = false;
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(c.host, from, c.bytes, cudaMemcpyDeviceToHost, stream);
-  }
+  for (const HostCopy& c : plain)
+    if (e == cudaSuccess) e = queue_copy(c, scratch, scratch_bytes, stream);
   if (block) {
     if (e == cudaSuccess) e = staged(device, stream, block, chunks, true);
     give_back(block);
   }
   const cudaError_t s = cudaStreamSynchronize(stream);
-  if (e == cudaSuccess) e = s;
-  if (e == cudaSuccess)
-    for (const HostCopy& c : plain)
-      if (c.fixed_point) host_fixed_to_double(c.host, c.bytes);
-  return e;
+  return e != cudaSuccess ? e : s;
 }
 
 cudaError_t copy_to_device(int device, cudaStream_t stream, void* target, const void* host, size_t bytes) {
   if (bytes == 0) return cudaSuccess;
-  Block* block = bytes >= kStagedCopyBytes && !page_locked(host) ? lease(device) : nullptr;
+  Block* block = nullptr;
+  if (bytes >= kStagedCopyBytes) {
+    bool locked = false;
+    const cudaError_t known = is_page_locked(host, bytes, &locked);
+    if (known != cudaSuccess) return known;
+    if (!locked) block = lease(device);
+  }
   if (block) {
     std::vector<Chunk> chunks;
     try {

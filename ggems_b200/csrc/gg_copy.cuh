@@ -30,9 +30,9 @@ struct HostCopy {
 constexpr size_t kStagedCopyBytes = 48u << 20;
 
 // Queues the copies on `stream` of `device` and waits for them.  The host
-// arrays may be pageable, page-locked or managed.  scratch: device memory that
-// fixed-point arrays up to its size are converted in (else page-locked ones by
-// the device in place, and others on the host).
+// arrays may be pageable, page-locked or managed, each as a whole
+// (cudaErrorInvalidValue if not).  scratch: device memory that fixed-point arrays
+// are converted in, piece by piece if it is smaller; needed where there are any.
 cudaError_t copies_to_host(int device, cudaStream_t stream, const HostCopy* copies, int count, void* scratch = nullptr,
                            size_t scratch_bytes = 0);
 // One copy to the device; returns when it has landed.

@@ -72,11 +72,44 @@ def test_energies_are_converted_on_the_way(n):
         assert q.dtype == np.int64 and q.any()
         want = q.astype(np.float64) / 4294967296.0
         assert np.array_equal(T.edep[0], want)
-        # page-locked arrays: written by the device
+        # page-locked arrays (200^3: in two pieces of the device's scratch)
         pinned = abi.Tallies([], [n ** 3], alloc=lambda k, t: torch.zeros(
             k, dtype={np.int32: torch.int32, np.float64: torch.float64}[t], pin_memory=True).numpy())
         ctx.read_tallies(pinned)
         assert np.array_equal(pinned.edep[0], want)
         assert np.array_equal(pinned.hit[0], T.hit[0]) and np.array_equal(pinned.edep_squared[0], T.edep_squared[0])
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("last", [False, True])
+def test_partly_page_locked_array_is_refused(last):
+    """An energy array of which one page only is page-locked: an error before
+    anything is written, and the context goes on working."""
+    import torch
+    from ggems_b200 import _native
+    sc = scenes.water_box_scene(n=64, voxel=2.0)
+    src = scenes.XRaySource(monoenergy=scenes.F(60.0) * scenes.KEV, aperture_deg=6.0)
+    page = 4096
+    ctx = _native.Context(0)
+    try:
+        _, T, _ = parity.run_gpu(ctx, sc, src, 20000)
+        raw = np.zeros(64 ** 3 * 8 + 2 * page, np.uint8)
+        at = -raw.ctypes.data % page
+        edep = raw[at:at + 64 ** 3 * 8].view(np.float64)
+        partly = abi.Tallies([], [64 ** 3])
+        partly.edep[0] = edep
+        partly._ek[0] = abi.ptr(edep, C.c_double)
+        locked = edep.ctypes.data + (edep.nbytes - page if last else 0)
+        rt = torch.cuda.cudart()
+        assert int(rt.cudaHostRegister(locked, page, 0)) == 0
+        try:
+            with pytest.raises(RuntimeError):
+                ctx.read_tallies(partly)
+            assert not edep.any()
+        finally:
+            assert int(rt.cudaHostUnregister(locked)) == 0
+        ctx.read_tallies(partly)
+        assert np.array_equal(edep, T.edep[0])
     finally:
         ctx.close()
