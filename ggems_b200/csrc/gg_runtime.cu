@@ -646,7 +646,10 @@ GG_API int gg_context_create(int32_t device_index, gg_context** context) {
   };
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) return cleanup(fail(GG_ERROR_CUDA, "stream"));
   if (cudaMalloc(&c->rng, 5 * S * sizeof(uint32_t)) != cudaSuccess) return cleanup(fail(GG_ERROR_OUT_OF_MEMORY, "rng"));
-  cudaMemset(c->rng, 0, 5 * S * sizeof(uint32_t));
+  // Cleared on the context's own stream, here and below: its work does not wait
+  // for the default stream's, and a label read before it is 0 would index past the tables.
+  if (cudaMemsetAsync(c->rng, 0, 5 * S * sizeof(uint32_t), c->stream) != cudaSuccess)
+    return cleanup(fail(GG_ERROR_CUDA, "rng"));
   float** fp[7] = {&c->particles.E, &c->particles.px, &c->particles.py, &c->particles.pz,
                    &c->particles.dx, &c->particles.dy, &c->particles.dz};
   for (auto f : fp)
@@ -655,7 +658,7 @@ GG_API int gg_context_create(int32_t device_index, gg_context** context) {
   if (cudaMalloc(&c->particles.status, S) != cudaSuccess || cudaMalloc(&c->particles.scatter, S) != cudaSuccess ||
       cudaMalloc(&c->particles.solid_id, S * sizeof(int32_t)) != cudaSuccess)
     return cleanup(fail(GG_ERROR_OUT_OF_MEMORY, "particles"));
-  if (cudaMalloc(&c->zero_label, 16) != cudaSuccess || cudaMemset(c->zero_label, 0, 16) != cudaSuccess)
+  if (cudaMalloc(&c->zero_label, 16) != cudaSuccess || cudaMemsetAsync(c->zero_label, 0, 16, c->stream) != cudaSuccess)
     return cleanup(fail(GG_ERROR_OUT_OF_MEMORY, "labels"));
   if (cudaMalloc(&c->slot_counter, sizeof(unsigned int)) != cudaSuccess ||
       cudaMalloc(&c->error, sizeof(int)) != cudaSuccess)
@@ -1546,7 +1549,7 @@ GG_API int gg_set_tracking(gg_context* c, int32_t slot, int32_t capacity) {
   if (slot < 0) return GG_OK;
   GG_CUDA(cudaMalloc(&c->tracking_points, static_cast<size_t>(capacity) * sizeof(gg_track_point)));
   GG_CUDA(cudaMalloc(&c->tracking_count, sizeof(int32_t)));
-  GG_CUDA(cudaMemset(c->tracking_count, 0, sizeof(int32_t)));
+  GG_CUDA(cudaMemsetAsync(c->tracking_count, 0, sizeof(int32_t), c->stream));
   c->tracking_slot = slot;
   c->tracking_capacity = capacity;
   return GG_OK;
