@@ -550,8 +550,14 @@ int make_dev_solid(gg_context* c, const gg_solid& g, gg::DevSolid* out, std::vec
   const uint32_t nx = static_cast<uint32_t>(g.number_of_voxels[0]), ny = static_cast<uint32_t>(g.number_of_voxels[1]);
   d.label_bias = 0x4b000000u * (nx * ny + nx + 1u);
   if (g.type == GG_SOLID_BOX) {
-    // the transport kernel takes it as a grid of one voxel of material 0
-    for (int a = 0; a < 3; ++a) d.number_of_voxels[a] = 1;
+    // The transport kernel takes it as a grid of one voxel of material 0, whose
+    // faces are the box's.  A box's voxel fields in gg_solid mean nothing and may
+    // hold anything: none reaches the kernel.
+    for (int a = 0; a < 3; ++a) {
+      d.number_of_voxels[a] = 1;
+      d.voxel_sizes[a] = d.inv_voxel_sizes[a] = 0.0f;
+    }
+    d.label_bias = 0;
     d.voxel_mode = gg::kVoxelBox;
   }
   std::memcpy(d.virtual_element_number, g.virtual_element_number, sizeof(d.virtual_element_number));

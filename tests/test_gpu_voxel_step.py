@@ -91,3 +91,28 @@ def test_short_steps_match_whole_ones(n, voxel, rotation, dose, aperture):
                 assert np.array_equal(getattr(T0, name)[0], getattr(T1, name)[0])
     finally:
         ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("value,count", [(float("nan"), 1), (float("inf"), 7), (-1.0e-30, -3)])
+def test_a_detector_box_has_no_voxels(value, count):
+    """gg_solid's voxel fields are a voxelized solid's: whatever a box holds there changes nothing."""
+    from ggems_b200 import _native
+    ctx = _native.Context(0)
+    try:
+        src = scenes.XRaySource(spectrum=scenes.synthetic_spectrum(), aperture_deg=9.0)
+        runs = []
+        for fill in (False, True):
+            sc = _scene(16, 8.0, [], False, 64)
+            if fill:
+                box = sc.solids[-1]
+                box.voxel_sizes[:] = [value] * 3
+                box.number_of_voxels[:] = [count] * 3
+            runs.append(parity.run_gpu(ctx, sc, src, 40000))
+        (P0, T0, st0), (P1, T1, st1) = runs
+        assert T0.histograms[0].sum() > 10000 and parity.history_agreement(P0, P1)[0] == 1.0
+        assert np.array_equal(st0, st1)
+        for a, b in zip(T0.histograms, T1.histograms):
+            assert np.array_equal(a, b)
+    finally:
+        ctx.close()
