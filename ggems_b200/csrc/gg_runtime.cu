@@ -1111,12 +1111,15 @@ int prepare_jobs(gg_context* c, const gg_job* jobs, int32_t n, std::vector<void*
   };
   for (int s = 0; s < c->number_of_solids; ++s) need_mode(c->solid_dev_host[s]);
   for (const gg::DevSolid& d : job_solids) need_mode(d);
+  // Every job's solids like the first job's: the navigator of each, and for a
+  // voxelized one everything that the voxel steps read before the labels.
   P.shared_grids = 1;
   for (size_t i = 0; i < job_solids.size(); ++i) {
-    // everything that the voxel steps read before the labels
+    const gg::DevSolid& job = job_solids[i];
     const gg::DevSolid& first = job_solids[i % c->number_of_solids];
-    if (job_solids[i].type == GG_SOLID_VOXELIZED || first.type == GG_SOLID_VOXELIZED)
-      P.shared_grids &= std::memcmp(&job_solids[i], &first, offsetof(gg::DevSolid, labels)) == 0 ? 1 : 0;
+    const bool voxels = job.type == GG_SOLID_VOXELIZED || first.type == GG_SOLID_VOXELIZED;
+    if (job.navigator != first.navigator || (voxels && std::memcmp(&job, &first, offsetof(gg::DevSolid, labels)) != 0))
+      P.shared_grids = 0;
   }
   P.three_processes = 1;
   for (uint32_t pack : c->process_pack) P.three_processes &= (pack & gg::kPackCount) == 3u ? 1 : 0;

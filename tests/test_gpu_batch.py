@@ -206,3 +206,42 @@ def test_launch_shape_does_not_change_results(ctx):
         ctx.set_tuning()
         ctx.set_launch()
         ctx.set_stash()
+
+
+def _mesh_job(path, navigators):
+    """A meshed body and a voxelized cube behind it, with these navigators (0 water, 1 bone)."""
+    sc = scenes.Scene()
+    water, bone = sc.add_tables(scenes.Tables(["Water"])), sc.add_tables(scenes.Tables(["Bone185"]))
+    assert (water, bone) == (0, 1)
+    sc.add_meshed(path, navigators[0], depth=3, dose={"dosel_size": (10.0, 10.0, 10.0)})
+    sc.add_voxelized(np.zeros((8, 8, 8), np.uint8), (10.0, 10.0, 10.0), navigators[1],
+                     ops=[("translation", (300.0, 0.0, 0.0))], dose={})
+    return sc, scenes.XRaySource(spectrum=scenes.synthetic_spectrum(), aperture_deg=6.0)
+
+
+@pytest.mark.parametrize("second", [(1, 0), (1, 1), (0, 1)])
+def test_jobs_with_other_navigators(ctx, tmp_path, second):
+    """A solid's navigator is the job's: the same states and tallies, bit for bit,
+    as the jobs one after another."""
+    from ggems_b200 import workloads
+    path = str(tmp_path / "body.stl")
+    v, f = workloads.icosphere(2)
+    workloads.write_stl(path, (v * 70.0)[f].astype(scenes.F))
+    scs = [_mesh_job(path, nav) for nav in ((0, 0), second)]
+    spec = _spec([(sc, src, 40000) for sc, src in scs])
+    out = []
+    for together in (True, False):
+        ctx.upload_scene(scs[0][0].struct())
+        ctx.set_random_states(scenes.seed_states(777))
+        for jobs in ([spec] if together else [[j] for j in spec]):
+            ctx.run_jobs(jobs)
+        T = scs[0][0].tallies()
+        ctx.read_tallies(T)
+        st = np.zeros((5, abi.GG_MAXIMUM_PARTICLES), np.uint32)
+        ctx.get_random_states(st)
+        out.append((T, st))
+    (T0, st0), (T1, st1) = out
+    assert T0.hit[0].sum() > 10000 and T0.hit[1].sum() > 100  # both solids are reached
+    assert np.array_equal(st0, st1)
+    for k in range(2):
+        assert np.array_equal(T0.edep[k], T1.edep[k]) and np.array_equal(T0.hit[k], T1.hit[k])
