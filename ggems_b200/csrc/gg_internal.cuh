@@ -29,18 +29,17 @@ constexpr int kBlockThreads = 256;  // default transport block size (the autotun
 // Fixed-point scale of the energy tally: edep is accumulated as int64 multiples of 2^-32 MeV.
 constexpr double kEdepScale = 4294967296.0;
 
-// Values for which the transport kernel's quotient() (reciprocal + fused
-// multiply-adds instead of a division) is proven: no overflow, no subnormal
-// remainder for the operands transport divides.
-constexpr float kQuotientMin = 1.0e-25f, kQuotientMax = 1.0e25f;
 constexpr uint32_t kPackCount = 0xffu;
-// Voxel index of a solid: general (divisions, integer conversions),
-// multiplication by an exact 2^-k, or quotient() with the correctly rounded
-// reciprocal; the last two for at most 2^22 voxels an axis (trunc by rounding
-// at 2^23) in a grid where the voxel step's short forms hold (fast_steps in
-// gg_runtime.cu).  A launch takes the first of general, reciprocal, pow2 that one
-// of its voxelized solids needs; general: whole steps only.  A box takes whole
-// steps too, as a grid of one voxel.
+// How a solid's voxel index divides by the voxel size.  General (divisions,
+// integer conversions): grids that fast_steps in gg_runtime.cu refuses.  The
+// others, whose axes it bounds to 2048 mm of voxels of at least 8 um (2^18
+// voxels): multiplication by an exact 2^-k, or quotient() with the correctly
+// rounded reciprocal.  A launch takes the first of general, reciprocal, pow2 that
+// one of its voxelized solids needs, and with general the kernel variants whose
+// voxel steps take any grid.  Those cost 14 to 16 % where the short forms would do
+// (1e7 primaries through 128^3 and 256^3 CT 20.1 against 17.3 ms and 27.5 against
+// 23.0 ms, 128^3 dose of 2e6 5.2 against 4.5 ms).  A box takes whole steps, as a
+// grid of one voxel.
 constexpr int kVoxelGeneral = 0, kVoxelPow2 = 1, kVoxelReciprocal = 2, kVoxelBox = 3;
 
 struct alignas(16) DevNavigator {
@@ -190,7 +189,7 @@ struct TransportParams {
   int32_t tracking_capacity;
   gg_track_point* tracking_points;
   int32_t* tracking_count;
-  int32_t voxel_mode;               // kVoxelGeneral, kVoxelReciprocal or kVoxelPow2: what serves every voxelized solid of the launch
+  int32_t voxel_mode;               // kVoxelGeneral, kVoxelReciprocal or kVoxelPow2: what serves every voxelized solid of the launch's jobs
   int32_t three_processes;          // every navigator has all three
   int32_t shared_grids;             // batched launch: every job's voxelized solids have the first job's grids
   int32_t photon_tracking;          // some dose map counts photons
@@ -227,8 +226,8 @@ struct DoseParams {
 
 void launch_transport(const TransportParams& p, int grid, int threads, size_t smem, void* stream, bool mesh, bool dose,
                       bool aux, int stash);
-cudaError_t configure_transport(size_t smem, int threads, int* blocks_per_sm, bool mesh, bool batch, bool dose, bool aux,
-                                int stash);
+cudaError_t configure_transport(const TransportParams& p, size_t smem, int threads, int* blocks_per_sm, bool mesh,
+                                bool dose, bool aux, int stash);
 cudaError_t set_rayleigh_fit(const float* pp);
 void launch_compute_dose(const DoseParams& p, void* stream);
 

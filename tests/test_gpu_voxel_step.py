@@ -1,10 +1,10 @@
-"""The transport kernel's short voxel step against its whole step.
+"""The transport kernel's short voxel step against its general forms.
 
 * surely_crosses() (CPU, float arithmetic): where it says that a photon crosses
   its voxel, no process's -logf(u) / sigma is below the distance, with the
   logarithm an ulp either way.
-* On the GPU a launch takes whole steps only when a grid of it is too long for
-  the short ones: the same histories, states and tallies bit for bit, for odd
+* On the GPU a launch takes the general index, clamp and distance when a grid of
+  it is too long for the short ones: the same histories, states and tallies bit for bit, for odd
   voxel counts, voxel sizes with and without a power of two, a rotated phantom,
   and a pencil beam along each axis of the grid.
 """
@@ -72,7 +72,7 @@ def _scene(n, voxel, ops, dose, far_voxels):
     (40, 2.5, (0.0, math.pi / 2, 0.0), False, 0.0),
     (1, 60.0, (0.0, 0.0, 0.0), True, 2.0),
 ])
-def test_short_steps_match_whole_ones(n, voxel, rotation, dose, aperture):
+def test_short_steps_match_the_general_forms(n, voxel, rotation, dose, aperture):
     from ggems_b200 import _native
     ctx = _native.Context(0)
     try:
