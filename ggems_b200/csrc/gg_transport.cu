@@ -1032,6 +1032,12 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
     if (why >= 2) end_history();
     else phase = kFind;
   };
+  // A detector box takes whole steps in the rare rounds: nearly all of them end
+  // in an interaction, and full warps sample those.  Against steps in the tracking
+  // loop, 5e6 primaries on a panel without a phantom: water 300 mm 4.06 -> 2.51 ms,
+  // 20 mm 2.35 -> 1.44, GOS 0.3 mm 1.09 -> 0.95, 10 mm at 140 keV 1.04 -> 0.97, but
+  // 10 mm at 120 kVp, which stops all in one step, 0.87 -> 0.93; 46 curved modules
+  // around a phantom, 2e7: 11.3 -> 9.0 ms.
   auto track_phase = [&](int type) {
     return type == GG_SOLID_VOXELIZED              ? kTrackVoxel
            : (kFull && type == GG_SOLID_MESHED) ? kTrackMesh
