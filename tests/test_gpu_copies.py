@@ -113,3 +113,25 @@ def test_partly_page_locked_array_is_refused(last):
         assert np.array_equal(edep, T.edep[0])
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("n", [0, 1, 1000, abi.GG_MAXIMUM_PARTICLES - 1, abi.GG_MAXIMUM_PARTICLES])
+def test_random_states_of_some_slots(n):
+    """The first n slots of the five arrays go up and come back; the others stay."""
+    from ggems_b200 import _native
+    S = abi.GG_MAXIMUM_PARTICLES
+    ctx = _native.Context(0)
+    try:
+        first, then = (np.random.default_rng(k).integers(0, 1 << 32, (5, S), dtype=np.uint32) for k in (1, 2))
+        ctx.set_random_states(first)
+        _native.check(_native.lib.gg_set_random_states(ctx.handle, abi.ptr(then, C.c_uint32), n))
+        want = first.copy()
+        want[:, :n] = then[:, :n]
+        back = np.zeros((5, S), np.uint32)
+        ctx.get_random_states(back)
+        assert np.array_equal(back, want)
+        some = np.zeros((5, S), np.uint32)
+        _native.check(_native.lib.gg_get_random_states(ctx.handle, abi.ptr(some, C.c_uint32), n))
+        assert np.array_equal(some[:, :n], want[:, :n]) and not some[:, n:].any()
+    finally:
+        ctx.close()
