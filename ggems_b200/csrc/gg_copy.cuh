@@ -38,8 +38,8 @@ cudaError_t copies_to_host(int device, cudaStream_t stream, const HostCopy* copi
 // One copy to the device; returns when it has landed.
 cudaError_t copy_to_device(int device, cudaStream_t stream, void* target, const void* host, size_t bytes);
 
-// The page-locked blocks (at most two of 8 MB per device, made on first use)
-// are kept while some object that copies holds them, and freed with the last.
+// The page-locked blocks (at most two of 8 MB per device, made once they pay) are
+// kept while some object that copies holds them, and freed with the last.
 void hold_staging(int device);
 void release_staging(int device);
 

@@ -19,6 +19,18 @@ STAGED = 48 << 20  # kStagedCopyBytes
 SIZES = [1, 524_289, STAGED - 1, STAGED, STAGED + 1, STAGED + 524_288, 70_000_001]
 
 
+@pytest.fixture(scope="module", autouse=True)
+def staging():
+    """A volume that stays, and copies enough for the staging block to be made and kept."""
+    from ggems_b200._native import Volume, check, lib
+    n = 256 << 20
+    src = np.zeros(n, np.uint8)
+    v = Volume(abi.GG_MET_UCHAR, (n, 1, 1), (1.0, 1.0, 1.0))
+    check(lib.gg_volume_upload(v.handle, C.c_void_p(src.ctypes.data), n))
+    yield
+    v.close()
+
+
 def _round_trip(n, seed, offset=0, pinned=False):
     from ggems_b200._native import Volume, check, lib
     rng = np.random.default_rng(seed)
@@ -135,3 +147,30 @@ def test_random_states_of_some_slots(n):
         assert np.array_equal(some[:, :n], want[:, :n]) and not some[:, n:].any()
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("mb", [50, 64, 300])
+def test_before_and_after_the_block_is_made(mb):
+    """In a process of its own: copies of one volume, the first ones by the
+    driver and the later ones through a block made meanwhile, and again after
+    the last holder has gone."""
+    import subprocess
+    import sys
+    code = """
+import ctypes as C, numpy as np
+from ggems_b200 import abi
+from ggems_b200._native import Volume, check, lib
+n = (%d << 20) + 5
+for again in range(2):
+    v = Volume(abi.GG_MET_UCHAR, (n, 1, 1), (1.0, 1.0, 1.0))
+    for k in range(5):
+        src = np.random.default_rng(10 * again + k).integers(0, 256, n, dtype=np.uint8)
+        check(lib.gg_volume_upload(v.handle, C.c_void_p(src.ctypes.data), n))
+        back = np.empty(n, np.uint8) if k %% 2 else np.zeros(n, np.uint8)
+        check(lib.gg_volume_download(v.handle, C.c_void_p(back.ctypes.data), n))
+        assert np.array_equal(src, back), (again, k)
+    v.close()
+print("ok")
+""" % mb
+    out = subprocess.run([sys.executable, "-c", code], cwd=scenes.ROOT, capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0 and "ok" in out.stdout, out.stderr
