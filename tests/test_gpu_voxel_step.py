@@ -4,9 +4,10 @@
   its voxel, no process's -logf(u) / sigma is below the distance, with the
   logarithm an ulp either way.
 * On the GPU a launch takes the general index, clamp and distance when a grid of
-  it is too long for the short ones: the same histories, states and tallies bit for bit, for odd
-  voxel counts, voxel sizes with and without a power of two, a rotated phantom,
-  and a pencil beam along each axis of the grid.
+  it is too long for the short ones: the same histories, states and tallies bit
+  for bit as with both short forms of the index, for odd voxel counts, voxel sizes
+  with and without a power of two, a rotated phantom, a pencil beam along each axis
+  of the grid, and with the track-length estimator.
 """
 
 import math
@@ -48,14 +49,26 @@ def test_a_sure_crossing_has_no_nearer_interaction(seed):
         assert ((a / sigma)[sure] >= distance[sure]).all()
 
 
-def _scene(n, voxel, ops, dose, far_voxels):
+# A solid far off the beam that decides the launch's form of the voxel step
+# (voxel size in mm along x, voxels): short with powers of two, short with
+# reciprocals, general (longer than the 2048 mm that the short forms take).
+FAR = {"pow2": (0.015625, 64), "reciprocal": (0.02, 64), "general": (0.02, 1 << 17)}
+
+
+def _forms(voxel):
+    """The forms that a grid of these voxels can be stepped through with."""
+    assert all((size * count > 2048.0) == (form == "general") and size > 0.008 for form, (size, count) in FAR.items())
+    assert all((math.frexp(size)[0] == 0.5) == (form == "pow2") for form, (size, _) in FAR.items())
+    return ["pow2"] * (math.frexp(voxel)[0] == 0.5) + ["reciprocal", "general"]
+
+
+def _scene(n, voxel, ops, dose, form, tle=False):
     sc = scenes.Scene()
     t = sc.add_tables(scenes.Tables(["Air", "Water", "Bone185"]))
     sc.add_voxelized(scenes.ellipsoid_phantom(n, voxel, seed=4), (voxel, voxel, voxel), t, ops=ops,
-                     dose={"photon_tracking": True} if dose else None)
-    # far off the beam; 1.28 mm long, or too long for the launch's short steps
-    far = np.ones((1, 1, far_voxels), np.uint8)
-    sc.add_voxelized(far, (0.02, 1.0, 1.0), t, ops=[("translation", (0.0, 5000.0, 0.0))])
+                     dose={"photon_tracking": True, "tle": tle} if dose else None)
+    size, count = FAR[form]
+    sc.add_voxelized(np.ones((1, 1, count), np.uint8), (size, 1.0, 1.0), t, ops=[("translation", (0.0, 5000.0, 0.0))])
     sc.add_flat_detector(sc.add_tables(scenes.Tables(["GOS"])), (50, 40, 1), (8.0, 10.0, 10.0), 1500.0, 1000.0,
                          F(10.0) * scenes.KEV)
     return sc
@@ -64,31 +77,40 @@ def _scene(n, voxel, ops, dose, far_voxels):
 @pytest.mark.gpu
 @pytest.mark.parametrize("n,voxel,rotation,dose,aperture", [
     (33, 4.0, (0.0, 0.0, 0.0), False, 9.0),
+    (40, 3.1, (0.0, 0.0, 0.0), False, 9.0),
     (64, 2.0, (0.0, 0.0, 0.0), True, 9.0),
+    (64, 2.0, (0.0, 0.0, 0.0), "tle", 9.0),
     (41, 3.1, (0.0, 0.0, 0.3), True, 9.0),
+    (41, 3.1, (0.0, 0.0, 0.3), "tle", 9.0),
     (117, 0.7, (0.2, 0.1, 0.0), False, 4.0),
     (40, 2.5, (0.0, 0.0, 0.0), True, 0.0),
     (40, 2.5, (0.0, 0.0, math.pi / 2), True, 0.0),
     (40, 2.5, (0.0, math.pi / 2, 0.0), False, 0.0),
     (1, 60.0, (0.0, 0.0, 0.0), True, 2.0),
+    (1, 64.0, (0.0, 0.0, 0.0), "tle", 2.0),
 ])
 def test_short_steps_match_the_general_forms(n, voxel, rotation, dose, aperture):
     from ggems_b200 import _native
     ctx = _native.Context(0)
     try:
         src = scenes.XRaySource(spectrum=scenes.synthetic_spectrum(), aperture_deg=aperture)
-        runs = [parity.run_gpu(ctx, _scene(n, voxel, [("rotation", rotation)], dose, far), src, 40000)
-                for far in (64, 1 << 17)]
-        (P0, T0, st0), (P1, T1, st1) = runs
+        runs = [parity.run_gpu(ctx, _scene(n, voxel, [("rotation", rotation)], dose, form, dose == "tle"), src, 40000)
+                for form in _forms(voxel)]
+        P0, T0, st0 = runs[0]
         assert T0.histograms[0].sum() > 0
-        assert parity.history_agreement(P0, P1)[0] == 1.0
-        assert np.array_equal(st0, st1)
-        for a, b in zip(T0.histograms, T1.histograms):
-            assert np.array_equal(a, b)
         if dose:
             assert T0.hit[0].sum() > 0
-            for name in ("edep", "hit", "photon_tracking"):
-                assert np.array_equal(getattr(T0, name)[0], getattr(T1, name)[0])
+        for P1, T1, st1 in runs[1:]:
+            assert parity.history_agreement(P0, P1)[0] == 1.0
+            assert np.array_equal(st0, st1)
+            for a, b in zip(T0.histograms, T1.histograms):
+                assert np.array_equal(a, b)
+            if dose:
+                for name in ("edep", "hit", "photon_tracking"):
+                    assert np.array_equal(getattr(T0, name)[0], getattr(T1, name)[0])
+                # a sum of doubles in any order: n terms, each within (n - 1) 2^-53 of the sum, n <= the hits
+                e = T0.edep_squared[0]
+                assert (np.abs(T1.edep_squared[0] - e) <= np.maximum(T0.hit[0], 1) * 2.0 ** -52 * e).all()
     finally:
         ctx.close()
 
@@ -103,7 +125,7 @@ def test_a_detector_box_has_no_voxels(value, count):
         src = scenes.XRaySource(spectrum=scenes.synthetic_spectrum(), aperture_deg=9.0)
         runs = []
         for fill in (False, True):
-            sc = _scene(16, 8.0, [], False, 64)
+            sc = _scene(16, 8.0, [], False, "pow2")
             if fill:
                 box = sc.solids[-1]
                 box.voxel_sizes[:] = [value] * 3
