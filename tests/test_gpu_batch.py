@@ -245,3 +245,28 @@ def test_jobs_with_other_navigators(ctx, tmp_path, second):
     assert np.array_equal(st0, st1)
     for k in range(2):
         assert np.array_equal(T0.edep[k], T1.edep[k]) and np.array_equal(T0.hit[k], T1.hit[k])
+
+
+@pytest.mark.parametrize("grids", [((32, 8.0), (32, 8.0)), ((33, 7.1), (33, 7.1)), ((32, 8.0), (64, 4.0)),
+                                   ((33, 7.1), (32, 8.0)), ((40, 6.0), (40, 6.5))])
+def test_voxel_grids_of_the_jobs(ctx, grids):
+    """Jobs with one grid (read from the first job's copy) and with grids of their
+    own: states and histograms bit for bit as the jobs one after another."""
+    phantoms = [(scenes.ellipsoid_phantom(n, voxel, seed=5 + k, n_bones=3), voxel) for k, (n, voxel) in enumerate(grids)]
+    jobs = _jobs(phantoms, [0.0, 77.0], 30000)
+    spec = _spec(jobs)
+    out = []
+    for together in (True, False):
+        ctx.upload_scene(jobs[0][0].struct())
+        ctx.set_random_states(scenes.seed_states(777))
+        for part in ([spec] if together else [[j] for j in spec]):
+            ctx.run_jobs(part)
+        T = jobs[0][0].tallies()
+        ctx.read_tallies(T)
+        st = np.zeros((5, abi.GG_MAXIMUM_PARTICLES), np.uint32)
+        ctx.get_random_states(st)
+        out.append((T, st))
+    (T0, st0), (T1, st1) = out
+    assert np.array_equal(st0, st1)
+    for a, b in zip(T0.histograms, T1.histograms):
+        assert a.sum() > 0 and np.array_equal(a, b)
