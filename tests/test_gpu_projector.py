@@ -31,7 +31,23 @@ def _chords(labels, mu, half, voxel, src, pixel):
     return float((mu[lab] * (t[1:] - t[:-1]) * ok).sum() * np.linalg.norm(d))
 
 
+def _along_a_face(src, d, half, voxel):
+    """Whether the ray runs nearly along an axis and, where it is in the grid, near a
+    voxel face or over one: rounding gives such a chord to either side."""
+    with np.errstate(divide="ignore", invalid="ignore"):
+        t = np.sort(np.array([(-half - src) / d, (half - src) / d]), axis=0)
+    along = np.abs(d) < 1e-3 * np.linalg.norm(d)
+    t_in, t_out = max(0.0, t[0][~along].max()), min(1.0, t[1][~along].min())
+    for a in np.flatnonzero(along):
+        k = (src[a] + np.array([t_in, t_out]) * d[a] + half[a]) / voxel[a]
+        if np.floor(k[0]) != np.floor(k[1]) or np.any(np.abs(k - np.round(k)) < 0.05):
+            return True
+    return False
+
+
 @pytest.mark.parametrize("elements,dims,voxel,count,inside", [
+    ((1, 1), (7, 7, 7), (8.0, 6.0, 5.0), 1, False),
+    ((33, 9), (31, 21, 11), (2.5, 3.0, 5.0), 1, False),
     ((33, 9), (12, 20, 7), (4.0, 3.0, 5.0), 1, False),
     ((1, 1), (5, 5, 5), (8.0, 8.0, 8.0), 3, False),
     ((64, 40), (31, 31, 31), (2.5, 2.5, 2.5), 5, False),
@@ -72,20 +88,21 @@ def test_projector_matches_chords(elements, dims, voxel, count, inside):
     assert np.array_equal(single, out[0, ..., 1])
     np.testing.assert_allclose(out[..., 0], np.exp(-out[..., 1]), rtol=2e-6)
     half = np.array([sc.solids[0].obb.border_max[a] for a in range(3)])
-    err, ref = [], []
+    err, ref, along_axis = [], [], 0
     for k in range(count):
         m = np.array(list(dets[k].obb.matrix), np.float64).reshape(4, 4)
         for j in range(elements[1]):
             for i in range(elements[0]):
-                # off-axis by the float rounding of the element's centre: rays on a
-                # voxel face belong to either side, so those are left out below
                 c = [dets[k].obb.border_min[0] + (i + 0.5) * size[0], dets[k].obb.border_min[1] + (j + 0.5) * size[1], 0, 1]
                 pixel = (m @ np.array(c))[:3]
                 d = pixel - srcs[k]
-                if k == 0 and np.min(np.abs(d)) < 1e-3 * np.linalg.norm(d):
-                    continue  # nearly along a face
+                if _along_a_face(srcs[k].astype(np.float64), d, half, np.array(voxel)):
+                    continue
+                along_axis += k == 0 and np.min(np.abs(d)) < 1e-3 * np.linalg.norm(d)
                 ref.append(_chords(labels, mu64, half, np.array(voxel), srcs[k].astype(np.float64), pixel))
                 err.append(out[k, j, i, 1] - ref[-1])
+    # odd voxel counts: the rays along an axis run through the voxels' middles
+    assert inside or along_axis > 0 or not all(n % 2 for n in dims[1:])
     err, ref = np.array(err), np.array(ref)
     # positions along the ray round to 2^-24 of its ~1500 mm length at each of up to
     # ~100 crossings: chords off by up to ~1e-2 mm x 0.06 mm^-1, 1e-3 of the rays' ~1
