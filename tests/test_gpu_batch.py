@@ -247,12 +247,20 @@ def test_jobs_with_other_navigators(ctx, tmp_path, second):
         assert np.array_equal(T0.edep[k], T1.edep[k]) and np.array_equal(T0.hit[k], T1.hit[k])
 
 
+@pytest.mark.parametrize("long_axis", [None, 0, 1])
 @pytest.mark.parametrize("grids", [((32, 8.0), (32, 8.0)), ((33, 7.1), (33, 7.1)), ((32, 8.0), (64, 4.0)),
                                    ((33, 7.1), (32, 8.0)), ((40, 6.0), (40, 6.5))])
-def test_voxel_grids_of_the_jobs(ctx, grids):
+def test_voxel_grids_of_the_jobs(ctx, grids, long_axis):
     """Jobs with one grid (read from the first job's copy) and with grids of their
-    own: states and histograms bit for bit as the jobs one after another."""
+    own: states and histograms bit for bit as the jobs one after another.
+    long_axis: this phantom is longer than the 2048 mm of the short voxel step, so the
+    launch takes the general forms, and the other phantom's job alone does not."""
     phantoms = [(scenes.ellipsoid_phantom(n, voxel, seed=5 + k, n_bones=3), voxel) for k, (n, voxel) in enumerate(grids)]
+    if long_axis is not None:
+        labels, voxel = phantoms[long_axis]
+        pad = int((2100.0 / voxel - labels.shape[0]) / 2)
+        phantoms[long_axis] = (np.pad(labels, ((pad, pad), (0, 0), (0, 0))), voxel)
+        assert phantoms[long_axis][0].shape[0] * voxel > 2048.0
     jobs = _jobs(phantoms, [0.0, 77.0], 30000)
     spec = _spec(jobs)
     out = []

@@ -116,6 +116,42 @@ def test_short_steps_match_the_general_forms(n, voxel, rotation, dose, aperture)
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("beside", ["world", "mesh", "no stash", "stash of 64 registers"])
+def test_other_kernels_of_the_general_forms(tmp_path, beside):
+    """The forms again in the kernels for a world grid, for a meshed solid and for other stashes."""
+    from ggems_b200 import _native, workloads
+    ctx = _native.Context(0)
+    try:
+        if "stash" in beside:
+            ctx.set_stash(registers=0 if beside == "no stash" else 64)
+        src = scenes.XRaySource(spectrum=scenes.synthetic_spectrum(), aperture_deg=6.0)
+        runs = []
+        for form in FAR:
+            sc = _scene(32, 4.0, [], True, form)
+            if beside == "world":
+                sc.set_world((20, 20, 20), (100.0, 100.0, 100.0))
+            if beside == "mesh":
+                path = str(tmp_path / "ball.stl")
+                v, f = workloads.icosphere(2)
+                workloads.write_stl(path, (v * 40.0)[f].astype(F))
+                sc.add_meshed(path, sc.add_tables(scenes.Tables(["Water"])), depth=3,
+                              ops=[("translation", (-300.0, 0.0, 0.0))], dose={"dosel_size": (10.0, 10.0, 10.0)})
+            runs.append(parity.run_gpu(ctx, sc, src, 40000))
+        P0, T0, st0 = runs[0]
+        assert T0.hit[0].sum() > 1000 and (beside != "mesh" or T0.hit[1].sum() > 1000)
+        for P1, T1, st1 in runs[1:]:
+            assert parity.history_agreement(P0, P1)[0] == 1.0 and np.array_equal(st0, st1)
+            for a, b in zip(T0.histograms + T0.edep + T0.hit, T1.histograms + T1.edep + T1.hit):
+                assert np.array_equal(a, b)
+            if beside == "world":
+                assert T0.world["photon_tracking"].sum() > 0
+                for name in ("photon_tracking", "energy", "momentum_x", "momentum_y", "momentum_z"):
+                    assert np.array_equal(T0.world[name], T1.world[name])
+    finally:
+        ctx.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("value,count", [(float("nan"), 1), (float("inf"), 7), (-1.0e-30, -3)])
 def test_a_detector_box_has_no_voxels(value, count):
     """gg_solid's voxel fields are a voxelized solid's: whatever a box holds there changes nothing."""
