@@ -1,14 +1,19 @@
 // Copies between device memory and the caller's host arrays.
 //
 // A copy from or to pageable memory runs through the driver's own staging on
-// one thread.  That is fast up to ~32 MB (16-18 GB/s on the measured host) and
-// slow beyond (11 GB/s up, 4.5 GB/s into pages not touched yet), where a copy is
-// bound by one core's page faults and moves.  Copies of kStagedCopyBytes or more
-// go through a block of page-locked slots instead: each of eight threads moves
-// chunks between its two slots and the caller's array while the copy engine fills
-// or drains the other one.  Measured, driver against staged: 134 MB up 12.0 / 5.2
-// ms, into new pages 29.9 / 8.3 ms; 64 MB 4.3 / 2.7 and 13.5 / 4.2 ms; 20 MB 1.04 /
-// 1.45 and 1.26 / 1.19 ms; 3 MB 0.25 / 0.26 and 0.21 / 0.38 ms.
+// one thread: 19 GB/s up to ~50 MB, 12 GB/s at 134 MB, and 4.7 GB/s into pages not
+// touched yet, where that thread takes the page faults.  Copies of kStagedCopyBytes or more go through a block of
+// page-locked slots instead: each of eight threads moves chunks between its two
+// slots and the caller's array while the copy engine fills or drains the other
+// one.  Measured, driver / staged with a block at hand (ms; medians):
+//
+//   MB                 16           24           32           47           134
+//   up                 0.87 / 1.39  1.29 / 1.69  1.70 / 2.10  2.56 / 2.58  11.2 / 5.5
+//   into touched pages 0.82 / 1.30  1.21 / 1.26  1.61 / 1.66  2.33 / 1.89  8.0 / 5.3
+//   into new pages     -            -            6.7 / 2.0    10.1 / 2.7   29 / 8
+//
+// (malloc hands out new pages from 32 MB on.)  48 MB is where both directions gain
+// whatever the pages; an array in new pages would gain from 32 MB on.
 #ifndef GG_COPY_CUH
 #define GG_COPY_CUH
 

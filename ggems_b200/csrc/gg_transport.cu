@@ -56,9 +56,11 @@ constexpr float kKissCorrection = -0x1.ffp-56f;  // -(2^-23 - 2^-32) * 2^-32, ex
 
 // Tracking steps a lane takes between two looks at its warp's waiting photons.
 // The look (ballots, counts, the stash's exchange test) costs every lane more
-// than a step; a lane that stops early idles for the rest.  5 / 8 / 12 / 20
-// steps: CBCT of 1e8 primaries 177 / 172 / 166 / 165 ms, 36 projections of 1e6
-// 27.6 / 26.9 / 26.4 / 26.3 ms, 64^3 dose of 1e6 1.84 / 1.81 / 1.83 / 1.76 ms.
+// than a step; a lane that stops early idles for the rest.  8 / 12 / 16 / 20 / 24
+// steps, the better of two runs: CBCT of 1e8 primaries 165.6 / 165.3 / 160.0 /
+// 156.7 / 155.5 ms, 36 projections of 1e6 27.2 / 26.2 / 26.0 / 25.2 / 24.6 ms, 64^3
+// dose of 1e6 1.66 / 1.67 / 1.65 / 1.62 / 1.63 ms; the two runs of one differ by up
+// to 5 %, so 16 and more are alike.
 constexpr int kTrackSteps = 16;
 constexpr float kTwo23 = 8388608.0f;
 
@@ -159,9 +161,7 @@ __device__ __forceinline__ bool in_aabb(V3 p, V3 mn, V3 mx) {
 // computes it there), so a direction's reciprocals can be computed once.
 // The reference's early returns all give kOutOfWorld and its running
 // tmin <= tmax test can only fail for good (tmin grows, tmax shrinks), so the
-// axes are combined without branches and tested once at the end.  (A branch for
-// the rare direction along a face instead of the selects: CBCT 33.7 against
-// 31.3 ms per 1e7 primaries.)
+// axes are combined without branches and tested once at the end.
 __device__ __forceinline__ float distance_to_aabb(V3 p, V3 d, V3 inv, V3 mn, V3 mx) {
   float tmin = FLT_MIN, tmax = FLT_MAX;
   bool miss = false;
@@ -880,14 +880,15 @@ __device__ __forceinline__ StashMask stash_mask(unsigned part, int h) {
 constexpr int transport_registers(int blocks) { return (65536 / (kBlockThreads * blocks)) & ~7; }
 
 // What bounds the kernel: the issue slots while photons cross large grids (CBCT
-// 256^3: 71 % of them busy), and instruction fetches where events are frequent
-// (36 projections through 64^3: 7 of the 17 cycles between two instructions of a
+// 256^3: 69 % of them busy), and instruction fetches where events are frequent
+// (36 projections through 64^3: 7.5 of the 14 cycles between two instructions of a
 // warp), since the warps of an SM are in different parts of the code.  So the
 // rare parts are kept short rather than fast: one copy of the exchange, of the
 // exit from a solid and of the azimuth after an interaction, loops that are not
-// unrolled, logarithms and exponentials out of line.  The samplers and the
-// sources went from 50 to 30 KB: CBCT of 1e8 229 -> 205 ms, 36 projections
-// 32.8 -> 28.8 ms, 64^3 dose 2.25 -> 2.09 ms.
+// unrolled, logarithms and exponentials out of line.  When the samplers and the
+// sources went from 50 to 30 KB, CBCT of 1e8 went from 229 to 205 ms, 36
+// projections from 32.8 to 28.8 and 64^3 dose from 2.25 to 2.09 ms (157 to 160, 26
+// and 1.65 ms with the short voxel step).
 //
 // kFull: the scene has a meshed solid, a world grid or a tracked particle;
 // kAux: the world walk and particle tracking are compiled in.  Scenes without
@@ -925,7 +926,8 @@ __global__ void __maxnreg__(transport_registers(kAux ? 2 : (kFull ? 3 : ((kBatch
   // run, the job's own array (global memory) in a batched launch.  Where all
   // jobs have the same grids (the angles of a scan), the voxel steps read those
   // from the shared-memory copy of the first job's: lanes in different jobs then
-  // read one address, not one each (36 projections of 1e6: 24.0 ms before).
+  // read one address, not one each (36 projections of 1e6: 27.6 ms without, 26.3
+  // with).
   const DevSolid* solids = scene_solids;
   int job = 0;
   const int number_of_jobs = kBatch ? P.number_of_jobs : 1;
